@@ -83,6 +83,7 @@ int resolve(const acg_params &p, SysDesc &d) {
   d.dof = 3.0 * (double)p.n - 3.0;  // DOF (MDcode/global.h:35)
   for (int i = 0; i < NHC_M; i++) d.q[i] = p.T * TAU_T * TAU_T;
   d.q[0] = d.dof * p.T * TAU_T * TAU_T;
+  for (int i = 0; i < NHC_M; i++) d.rq[i] = 1.0 / d.q[i];
   for (int i = 0; i < NHC_M; i++) d.q_baro[i] = p.T * TAU_P * TAU_P;
   d.w_eps = d.dof * p.T * TAU_P * TAU_P;
   for (int t = 0; t < 3; t++) {
@@ -1523,6 +1524,7 @@ int acg_set_temperature(acg_engine *e, int sys, double T) {
   d.T = T;
   for (int i = 0; i < NHC_M; i++) d.q[i] = T * TAU_T * TAU_T;
   d.q[0] = d.dof * T * TAU_T * TAU_T;
+  for (int i = 0; i < NHC_M; i++) d.rq[i] = 1.0 / d.q[i];
   for (int i = 0; i < NHC_M; i++) d.q_baro[i] = T * TAU_P * TAU_P;
   d.w_eps = d.dof * T * TAU_P * TAU_P;
   CK(cudaMemcpyAsync(e->d_desc + sys, &d, sizeof(SysDesc), cudaMemcpyHostToDevice, e->stream));

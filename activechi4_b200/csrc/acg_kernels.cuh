@@ -1019,32 +1019,58 @@ __device__ __forceinline__ void pair_fp32(PairAcc &a, const double4 &pi, int ti,
   }
 }
 
-// finish one system after its last force block: fixed-order sums, then the
-// thermostat chain (runs in a single block)
-__device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, int mode, double pe, double vir, double ke, double va);
+__device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, SysDesc &dbox, int mode, double pe, double vir,
+                                           double ke, double va);
 
+// copy of a structure by all threads of the block, in 8-byte words
+template <class T>
+__device__ __forceinline__ void copy_struct(T *dst, const T *src) {
+  static_assert(sizeof(T) % 8 == 0, "copied in 8-byte words");
+  const unsigned long long *a = reinterpret_cast<const unsigned long long *>(src);
+  unsigned long long *b = reinterpret_cast<unsigned long long *>(dst);
+  for (int k = threadIdx.x; k < (int)(sizeof(T) / 8); k += blockDim.x) b[k] = a[k];
+}
+
+// finish one system after its last force block: fixed-order sums, then the
+// thermostat chain (runs in a single block).  The system's state and
+// descriptor are copied to shared memory beside the partial sums (one round
+// trip to L2) and the state is written back whole, so the one thread that
+// runs the chain waits for no memory.
 __device__ void finalize_system(const View &v, int r, int mode) {
-  __shared__ double sh[32];
-  const SysDesc &d = v.desc[r];
-  SysState &st = v.st[r];
-  double pe = 0.0, vir = 0.0, ke = 0.0, va = 0.0;
-  const bool per_particle = d.box;
-  const int nparts = per_particle ? d.n : d.ntile_b;
+  __shared__ double sh[4][32];
+  __shared__ SysState ss;
+  __shared__ SysDesc sd;
+  SysDesc &dg = const_cast<SysDesc &>(v.desc[r]);
+  copy_struct(&ss, &v.st[r]);
+  copy_struct(&sd, &v.desc[r]);
+  double q[4] = {0.0, 0.0, 0.0, 0.0};
+  const bool per_particle = dg.box;
+  const int nparts = per_particle ? dg.n : dg.ntile_b;
   for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
-    const double2 *pp = per_particle ? reinterpret_cast<const double2 *>(&v.pacc[d.poff + k])
-                                     : reinterpret_cast<const double2 *>(&v.part_b[d.tile0_b + k]);
+    const double2 *pp = per_particle ? reinterpret_cast<const double2 *>(&v.pacc[dg.poff + k])
+                                     : reinterpret_cast<const double2 *>(&v.part_b[dg.tile0_b + k]);
     const double2 p0 = __ldcg(pp), p1 = __ldcg(pp + 1);
-    pe += p0.x;
-    vir += p0.y;
-    ke += p1.x;
-    va += p1.y;
+    q[0] += p0.x;
+    q[1] += p0.y;
+    q[2] += p1.x;
+    q[3] += p1.y;
   }
-  pe = block_sum_dyn(pe, sh);
-  vir = block_sum_dyn(vir, sh);
-  ke = block_sum_dyn(ke, sh);
-  va = block_sum_dyn(va, sh);
-  if (threadIdx.x != 0) return;
-  finalize_sums(d, st, mode, pe, vir, ke, va);
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
+  for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+    for (int k = 0; k < 4; k++) q[k] += __shfl_down_sync(0xffffffffu, q[k], o);
+  if (l == 0)
+    for (int k = 0; k < 4; k++) sh[k][w] = q[k];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int i = 0; i < nw; i++)
+      for (int k = 0; k < 4; k++) t[k] += sh[k][i];
+    finalize_sums(sd, ss, dg, mode, t[0], t[1], t[2], t[3]);
+    ss.counter_b = 0;
+  }
+  __syncthreads();
+  copy_struct(&v.st[r], &ss);
 }
 
 // thermostat and scalars of one system from its sums (one thread): pe and
@@ -1055,7 +1081,7 @@ __device__ void finalize_system(const View &v, int r, int mode) {
 // (MDcode/time_evolve.c:499-501), a ramp step's rescale to the ramp target
 // (adjustInitialTemp, MDcode/initialise.c:141-151, with inst_T of
 // calculate_temp, :153-164), or none (NVE)
-__device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, double kb) {
+__device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, SysDesc &dbox, double kb) {
   if (st.ramp_left > 0) {
     const double inst = 2.0 * (kb * 0.5) / d.dof;
     st.s1 = sqrt(st.ramp_T / inst);
@@ -1065,7 +1091,7 @@ __device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, dou
       eta[k] = st.eta_end[k];
       pet[k] = st.p_eta_end[k];
     }
-    double s1 = nhc_half(eta, pet, d.q, d.T, d.dof, d.dt, kb);
+    double s1 = nhc_half(eta, pet, d.q, d.rq, d.T, d.dof, d.dt, kb);
     for (int k = 0; k < NHC_M; k++) {
       st.eta_cur[k] = eta[k];
       st.p_eta_cur[k] = pet[k];
@@ -1078,7 +1104,6 @@ __device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, dou
     // U2 factors, then U1's box change eps += dt p_eps / w_eps, L = L0 exp(eps)
     // (:680-683); the drift keeps inv_L of the boundary length
     // (UpdateBoxForNPT ran at the end of the previous step)
-    SysDesc &dm = const_cast<SysDesc &>(d);
     double eta[NHC_M], pet[NHC_M], etab[NHC_M], petb[NHC_M];
     for (int k = 0; k < NHC_M; k++) {
       eta[k] = st.eta_end[k];
@@ -1106,9 +1131,9 @@ __device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, dou
     st.p_eps_cur = p_eps;
     st.eps_cur = eps;
     st.s1 = s1;
-    dm.invL = 1.0 / Lb;
-    dm.L = Ln;
-    dm.density = (double)d.n / (Ln * Ln * Ln);
+    dbox.invL = 1.0 / Lb;
+    dbox.L = Ln;
+    dbox.density = (double)d.n / (Ln * Ln * Ln);
     if (!(Ln > 0.0) || (int)((double)(int)Ln / d.cell_cut) != d.nc) st.status = 2;
   } else if (d.thermostat == 3) {
     // Gaussian isokinetic: the factors need sums of p.F and F^2 over the
@@ -1121,15 +1146,12 @@ __device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, dou
   }
 }
 
-__device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, int mode, double pe, double vir, double ke, double va) {
+__device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, SysDesc &dbox, int mode, double pe, double vir,
+                                           double ke, double va) {
   st.pe = 0.5 * pe;
   st.virial = (0.5 * vir) / 3.0;
   st.vir_act = va;
-  if (mode >= 2) {  // force evaluation only (calculate_forces)
-    __threadfence();
-    st.counter_b = 0;
-    return;
-  }
+  if (mode >= 2) return;  // force evaluation only (calculate_forces)
   double kb;
   if (mode == 0 && st.ramp_left > 0) {
     // a ramp step (advance_time_NVEFrog inside coldstart / breakxal): NVE, the
@@ -1200,7 +1222,7 @@ __device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, int m
         eta[k] = st.eta_cur[k];
         pet[k] = st.p_eta_cur[k];
       }
-      double s2 = nhc_half(eta, pet, d.q, d.T, d.dof, d.dt, ke);
+      double s2 = nhc_half(eta, pet, d.q, d.rq, d.T, d.dof, d.dt, ke);
       for (int k = 0; k < NHC_M; k++) {
         st.eta_end[k] = eta[k];
         st.p_eta_end[k] = pet[k];
@@ -1221,12 +1243,10 @@ __device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, int m
     kb = ke;
   }
   st.ke_end = kb * 0.5;
-  next_first_half(d, st, kb);
+  next_first_half(d, st, dbox, kb);
   if (mode == 0 && d.thermostat == 3 && st.gmode == 2) st.gmode = 1;
   if (!(ke == ke) || ke > 1.0e300) st.status = 1;
   st.prime = 0;
-  __threadfence();
-  st.counter_b = 0;
 }
 
 // ---------------------------------------------------------------------------
@@ -1310,7 +1330,7 @@ __global__ void __launch_bounds__(BLOCK_A) k_drift_apply(View v) {
   for (int b = 0; b < d.ntile_a; b++) kb += __ldcg(v.part_o + (size_t)(d.tile0_a + b) * OBS_EMAX * OBS_NV + 3);
   st.s2 = 1.0;
   st.ke_end = kb * 0.5;
-  next_first_half(d, st, kb);
+  next_first_half(d, st, const_cast<SysDesc &>(v.desc[r]), kb);
   st.drift = 0;
   __threadfence();
   st.counter_d = 0;
@@ -1601,7 +1621,7 @@ __global__ void __launch_bounds__(1024) k_rescale(View v, int r, double T) {
   if (threadIdx.x == 0) {
     st.s2 = 1.0;
     st.ke_end = k3 * 0.5;
-    next_first_half(d, st, k3);
+    next_first_half(d, st, const_cast<SysDesc &>(v.desc[r]), k3);
   }
 }
 
@@ -1616,7 +1636,7 @@ __global__ void k_ramp_begin(View v, int r, double T0, double dT, double T_end, 
   st.ramp_end = T_end;
   st.ramp_left = K;
   st.ramp_real = K;
-  next_first_half(d, st, 2.0 * st.ke_end);
+  next_first_half(d, st, const_cast<SysDesc &>(v.desc[r]), 2.0 * st.ke_end);
 }
 
 // lengthen system r's armed ramp to `total` steps; the steps after the ramp
@@ -3482,7 +3502,7 @@ __global__ void k_unload(View v, int r) {
 // recompute the next step's first thermostat half after a host change of the
 // chain or temperature (single thread per system)
 __global__ void k_prehalf(View v, int r) {
-  if (threadIdx.x == 0) next_first_half(v.desc[r], v.st[r], 2.0 * v.st[r].ke_end);
+  if (threadIdx.x == 0) next_first_half(v.desc[r], v.st[r], const_cast<SysDesc &>(v.desc[r]), 2.0 * v.st[r].ke_end);
 }
 
 __global__ void k_shuffle_now(View v, int r) { shuffle_component(v, r, blockIdx.x, v.st[r].step); }
