@@ -15,7 +15,7 @@ LIB = os.path.join(PKG, "libactivechi4_b200.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 SOURCES = ["acg_engine.cu", "acg_noalloc.cu"]
-HEADERS = ["acg_device.cuh", "acg_kernels.cuh"]
+HEADERS = ["acg_device.cuh", "acg_kernels.cuh", "acg_run.cuh"]
 
 
 def _nvcc() -> str:

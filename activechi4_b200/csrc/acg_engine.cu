@@ -13,7 +13,7 @@
 #include <vector>
 
 #include "../../include/activechi4.h"
-#include "acg_kernels.cuh"
+#include "acg_run.cuh"
 
 using namespace acg;
 
@@ -35,6 +35,7 @@ int fail(int code, const std::string &msg) {
 
 constexpr double TAU_T = 0.20;  // MDcode/time_evolve.c:477
 constexpr int GRAPH_STEPS = 32;
+constexpr int RUN_STEPS = 2048;       // most steps of one k_run_box launch (tens of ms)
 constexpr int BENCH_MAX_GRAPH = 256;  // acg_bench_steps: one graph for up to this many steps
 
 struct Layout {
@@ -223,6 +224,7 @@ int plan(const acg_params *params, int nsys, Layout &lay, int nsm) {
   add(4 * ((size_t)lay.nsub + 1));        // ssub
   add(4 * (2 * (size_t)nsys + 2));        // rbs
   add(4 * 2 * (size_t)MT_WORDS * nsys);   // mt
+  add(4 * (size_t)nsys);                  // run_order
   lay.bytes = b;
   return ACG_OK;
 }
@@ -243,6 +245,12 @@ struct acg_engine {
   SysDesc *d_desc = nullptr;
   int tpp = 4, block = 128, gtpp = 2, btpp = 2;  // btpp: whole-box kernels
   int ntiles_a = 0, ntiles_b = 0, ntiles_l = 0, ntiles_c = 0, ntiles_g = 0, ntiles_x = 0, ntiles_lc = 0;
+  // whole runs in one launch (k_run_box): blocks per cluster (0: the engine
+  // steps kernel by kernel), threads per block, state in shared memory, dynamic
+  // shared memory, systems in launch order (device)
+  int run_c = 0, run_nt = 0, run_resident = 0;
+  size_t run_smem = 0;
+  int *run_order = nullptr;
   int2 *d_tiles_b = nullptr;
   int2 *d_tiles_x = nullptr;
   std::vector<int> dirty;  // systems whose forces/lists must be recomputed
@@ -323,6 +331,78 @@ ForceFn force_fn(int tpp, int prec) {
   }
 #undef F
   return nullptr;
+}
+
+// ---- whole runs in one launch ----------------------------------------------
+using RunFn = void (*)(View, const int *, int, unsigned);
+template <int PREC, int NT, bool RES>
+RunFn run_fn_of(int tpp) {
+  switch (tpp) {
+    case 1: return k_run_box<1, PREC, NT, RES>;
+    case 2: return k_run_box<2, PREC, NT, RES>;
+    case 4: return k_run_box<4, PREC, NT, RES>;
+  }
+  return nullptr;
+}
+RunFn run_fn(int tpp, int prec, int nt, bool resident) {
+  if (!prec) return resident ? run_fn_of<0, 512, true>(tpp) : run_fn_of<0, 512, false>(tpp);
+  if (resident) return run_fn_of<1, 512, true>(tpp);
+  return nt == 512 ? run_fn_of<1, 512, false>(tpp) : run_fn_of<1, 1024, false>(tpp);
+}
+
+// whether one system can run inside a cluster: whole-box lists from sub-cells,
+// an integrator whose step is a kick/drift and one force pass, no uniform
+// direction shuffle
+bool run_eligible(const SysDesc &d) { return d.box && d.msub >= 5 && d.thermostat <= 2 && d.shuffle != 2; }
+
+// Cluster size, threads and shared memory of an engine's runs; run_c stays 0
+// where a system is not eligible or does not fit.  As many blocks per cluster
+// as leave every system its own cluster on the chip at once (7 of 16 blocks,
+// 15 of 8, 33 of 4, 74 of 2 with one block per SM), then one block per system.
+void plan_run(acg_engine *e, size_t smem_limit) {
+  const Layout &L = e->lay;
+  e->run_c = 0;
+  for (int r = 0; r < L.nsys; r++)
+    if (!run_eligible(L.desc[r])) return;
+  const int C = L.nsys <= 7 ? 16 : (L.nsys <= 15 ? 8 : (L.nsys <= 33 ? 4 : (L.nsys <= 74 ? 2 : 1)));
+  const int prec = L.desc[0].precision;
+  for (int resident = 1; resident >= 0; resident--) {
+    size_t least = 0, want = 0;
+    int nloc = 0;
+    for (int r = 0; r < L.nsys; r++) {
+      const SysDesc &d = L.desc[r];
+      const RunPlan p = run_plan(d.n, d.ncell, d.msub, prec, C, resident);
+      least = std::max(least, p.least());
+      // and the lists of the block's slots, about 120 entries of two bytes each
+      want = std::max(want, p.pool + p.stage_bytes + 256 * (size_t)p.nloc + p.perm_bytes);
+      nloc = std::max(nloc, p.nloc);
+    }
+    if (least > smem_limit) continue;
+    e->run_c = C;
+    e->run_resident = resident;
+    e->run_smem = std::min(smem_limit, std::max(least, want));
+    // FP64 pair terms take about 120 registers a thread
+    e->run_nt = prec && !resident && nloc * 2 > 512 ? 1024 : 512;
+    return;
+  }
+}
+
+// nsteps steps of every system, one cluster each
+int launch_run(acg_engine *e, int nsteps) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(e->lay.nsys * e->run_c);
+  cfg.blockDim = dim3(e->run_nt);
+  cfg.dynamicSmemBytes = e->run_smem;
+  cfg.stream = e->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = e->run_c;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, run_fn(e->btpp, e->lay.desc[0].precision, e->run_nt, e->run_resident), e->v,
+                        (const int *)e->run_order, nsteps, (unsigned)e->run_smem));
+  return ACG_OK;
 }
 
 // whole-box tiles: d.cpb cells of one system per block, the blocks of the
@@ -1017,6 +1097,7 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
   v.ssub = (int *)take(4 * ((size_t)L.nsub + 1));
   v.rbs = (int *)take(4 * (2 * (size_t)nsys + 2));
   v.mt = (unsigned int *)take(4 * 2 * (size_t)MT_WORDS * nsys);
+  e->run_order = (int *)take(4 * (size_t)nsys);
   v.tiles_a = ta;
   v.tiles_b = e->d_tiles_b;
   v.tiles_l = tl;
@@ -1036,6 +1117,7 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
   }
 
   std::vector<int2> h_a, h_l, h_c, h_g, h_lc;
+  std::vector<int> run_order;
   for (int r = 0; r < nsys; r++) {
     SysDesc &d = e->lay.desc[r];
     d.tile0_a = (int)h_a.size();
@@ -1102,6 +1184,19 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need) == cudaSuccess;
   };
   bool attr_ok = true;
+  plan_run(e, RUN_SMEM_MAX);
+  if (e->run_c) {
+    std::vector<int> ord(nsys);
+    for (int r = 0; r < nsys; r++) ord[r] = r;
+    std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return L.desc[a].n > L.desc[b].n; });
+    run_order.swap(ord);
+    for (int gt : {1, 2, 4}) {
+      const void *fn = (const void *)run_fn(gt, L.desc[0].precision, e->run_nt, e->run_resident);
+      attr_ok = attr_ok && raise_smem(fn, e->run_smem);
+      if (e->run_c > 8)
+        attr_ok = attr_ok && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+    }
+  }
   for (int gt : {1, 2, 4})
     for (int pr : {0, 1}) attr_ok = attr_ok && raise_smem((const void *)group_fn(gt, pr), group_smem(v.gcap));
   attr_ok = attr_ok && raise_smem((const void *)k_build_list_groups, list_smem(v.gcap));
@@ -1140,6 +1235,9 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
            cudaSuccess) ||
       (!h_l.empty() &&
        cudaMemcpyAsync(tl + h_lc.size(), h_l.data(), h_l.size() * sizeof(int2), cudaMemcpyHostToDevice,
+                       e->stream) != cudaSuccess) ||
+      (!run_order.empty() &&
+       cudaMemcpyAsync(e->run_order, run_order.data(), run_order.size() * sizeof(int), cudaMemcpyHostToDevice,
                        e->stream) != cudaSuccess) ||
       build_tiles_x(e) != ACG_OK)
     return cleanup_fail(fail(ACG_ERR_CUDA, "initial upload failed"));
@@ -1568,6 +1666,14 @@ int acg_compute_forces(acg_engine *e) {
 // nsteps steps in graph launches (no drift removal due inside them)
 int step_graphs(acg_engine *e, int nsteps) {
   int rc;
+  if (e->run_c) {
+    // launches of bounded length, so other engines' work gets the SMs between them
+    for (int left = nsteps; left > 0; left -= std::min(left, RUN_STEPS)) {
+      rc = launch_run(e, std::min(left, RUN_STEPS));
+      if (rc) return rc;
+    }
+    return ACG_OK;
+  }
   if (!e->no_while) {
     // device loop: one launch for the GRAPH_STEPS-step blocks, one for the rest
     const long long q = nsteps / GRAPH_STEPS, r = nsteps % GRAPH_STEPS;
@@ -1631,7 +1737,7 @@ int acg_prepare(acg_engine *e) {
   CK(cudaSetDevice(e->device));
   int rc = prime(e);
   if (rc) return rc;
-  if (e->no_while) return ACG_OK;
+  if (e->no_while || e->run_c) return ACG_OK;
   for (int k = 0; k < 3 && !e->no_while; k++)
     if (!e->wexec[k] &&
         build_while_graph(e, k < 2 ? GRAPH_STEPS : 1, e->counts + k, &e->wgraph[k], &e->wexec[k]) != ACG_OK)
@@ -1995,7 +2101,7 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
   for (const auto &reg : pieces)
     for (const auto &pc : reg) {
       const int K = (int)pc.first;
-      if (e->bench.count(K)) continue;
+      if (e->run_c || e->bench.count(K)) continue;
       cudaGraph_t g;
       cudaGraphExec_t x;
       rc = build_graph(e, K, &g, &x);
@@ -2019,12 +2125,18 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
   const size_t nl = plan.size();
   std::vector<cudaEvent_t> ev(2 * nl);
   for (auto &x : ev) CK(cudaEventCreate(&x));
-  long long ndrift = 0;
+  long long ndrift = 0, nrun = 0;
   for (size_t c = 0; c < nl; c++) {
     if (flush_bytes) CK(cudaMemsetAsync(e->flush, (int)(c & 0xff), flush_bytes, e->stream));
     CK(cudaEventRecord(ev[2 * c], e->stream));
     for (const auto &pc : pieces[c]) {
-      CK(cudaGraphLaunch(e->bench[(int)pc.first].second, e->stream));
+      if (e->run_c) {
+        rc = launch_run(e, (int)pc.first);
+        if (rc) return rc;
+        nrun++;
+      } else {
+        CK(cudaGraphLaunch(e->bench[(int)pc.first].second, e->stream));
+      }
       if (pc.second) {
         rc = launch_drift(e);
         if (rc) return rc;
@@ -2045,6 +2157,10 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
   CK(cudaMemcpy(st1.data(), e->v.st, sizeof(SysState) * nsys, cudaMemcpyDeviceToHost));
   *ms = tot;
   if (!launches) return ACG_OK;
+  if (e->run_c) {  // whole runs in one launch, and the drift removals
+    *launches = nrun + 2 * ndrift;
+    return ACG_OK;
+  }
   // kernels launched in the timed region: every step the kick/drift kernel
   // and each force kernel in use; a step whose switch takes the rebuild the
   // rebuild kernels with a non-empty grid, the shuffle the shuffle kernel,

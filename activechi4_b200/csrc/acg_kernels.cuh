@@ -153,10 +153,9 @@ __device__ __forceinline__ void mt_twist(unsigned int *mt) {
 // one component of one system (blockDim.x == BLOCK_SHUF); state read from
 // mt_in, the final state (after 3 nact draws) written to mt_out by comp 2
 __device__ void shuffle_ref_component(const View &v, int r, int comp, const unsigned int *mt_in,
-                                      unsigned int *mt_out) {
+                                      unsigned int *mt_out, signed char *s_k) {
   __shared__ unsigned int s_mt[MT_N];
   __shared__ int s_j[MT_N];
-  extern __shared__ signed char s_k[];
   const SysDesc &d = v.desc[r];
   const int nact = d.nact;
   char4 *kd = v.kdir + d.aoff;
@@ -221,9 +220,10 @@ __global__ void __launch_bounds__(BLOCK_SHUF) k_shuffle_ref(View v, int only) {
   const int r = only >= 0 ? only : (int)blockIdx.x / 3, comp = (int)blockIdx.x % 3;
   const SysDesc &d = v.desc[r];
   const SysState &st = v.st[r];
+  extern __shared__ signed char s_k[];
   if (d.nact == 0 || (only < 0 && !st.shuf)) return;
   unsigned int *mt = v.mt + (size_t)r * 2 * MT_WORDS;
-  shuffle_ref_component(v, r, comp, mt + (size_t)st.mt_cur * MT_WORDS, mt + (size_t)(st.mt_cur ^ 1) * MT_WORDS);
+  shuffle_ref_component(v, r, comp, mt + (size_t)st.mt_cur * MT_WORDS, mt + (size_t)(st.mt_cur ^ 1) * MT_WORDS, s_k);
 }
 
 // the stored state after a shuffle outside the step becomes current
@@ -304,7 +304,9 @@ __device__ __forceinline__ double brown_correct_one(const View &v, const SysDesc
 // U3 U2 (pending thermostat scales and the half kick) and U1 for one
 // particle, in the reference's order of roundings; returns |x_u - x_old|^2
 // (reduced units) for the rebuild test
-__device__ __forceinline__ double kick_drift_one(const View &v, const SysDesc &d, const SysState &st, int i) {
+// (V: the View, or a struct with the same per-slot arrays elsewhere)
+template <class V>
+__device__ __forceinline__ double kick_drift_one(const V &v, const SysDesc &d, const SysState &st, int i) {
   const double hdt = d.half_dt, dt = d.dt, il = d.invL;
   const double s1 = st.s1, s2 = st.s2;
   double px, py, pz;
@@ -1031,42 +1033,77 @@ __device__ __forceinline__ void copy_struct(T *dst, const T *src) {
   for (int k = threadIdx.x; k < (int)(sizeof(T) / 8); k += blockDim.x) b[k] = a[k];
 }
 
+// Per-system sums of a whole-box system, in an order that depends on its slots
+// alone (not on the kernel, its blocks or its threads per particle): segments
+// of 32 slots added up as a butterfly tree over slot bits 0 to 4, then the
+// segments, one warp: lane l takes segments l, l + 32, ... and the lanes are
+// added up as a butterfly.
+__device__ __forceinline__ double4 add4(const double4 &a, const double4 &b) {
+  return make_double4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w);
+}
+__device__ __forceinline__ double4 xor4(const double4 &a, int o) {
+  return add4(a, make_double4(__shfl_xor_sync(0xffffffffu, a.x, o), __shfl_xor_sync(0xffffffffu, a.y, o),
+                              __shfl_xor_sync(0xffffffffu, a.z, o), __shfl_xor_sync(0xffffffffu, a.w, o)));
+}
+__device__ __forceinline__ double4 total_of_segments(const double4 *seg, int nseg) {
+  double4 t = make_double4(0.0, 0.0, 0.0, 0.0);
+  for (int g = threadIdx.x & 31; g < nseg; g += 32) t = add4(t, seg[g]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t = xor4(t, o);
+  return t;
+}
+
 // finish one system after its last force block: fixed-order sums, then the
 // thermostat chain (runs in a single block).  The system's state and
 // descriptor are copied to shared memory beside the partial sums (one round
 // trip to L2) and the state is written back whole, so the one thread that
-// runs the chain waits for no memory.
-__device__ void finalize_system(const View &v, int r, int mode) {
+// runs the chain waits for no memory.  seg: shared memory for a whole-box
+// system's segment sums (32 bytes per 32 slots).
+__device__ void finalize_system(const View &v, int r, int mode, double4 *seg) {
   __shared__ double sh[4][32];
   __shared__ SysState ss;
   __shared__ SysDesc sd;
   SysDesc &dg = const_cast<SysDesc &>(v.desc[r]);
   copy_struct(&ss, &v.st[r]);
   copy_struct(&sd, &v.desc[r]);
-  double q[4] = {0.0, 0.0, 0.0, 0.0};
-  const bool per_particle = dg.box;
-  const int nparts = per_particle ? dg.n : dg.ntile_b;
-  for (int k = threadIdx.x; k < nparts; k += blockDim.x) {
-    const double2 *pp = per_particle ? reinterpret_cast<const double2 *>(&v.pacc[dg.poff + k])
-                                     : reinterpret_cast<const double2 *>(&v.part_b[dg.tile0_b + k]);
-    const double2 p0 = __ldcg(pp), p1 = __ldcg(pp + 1);
-    q[0] += p0.x;
-    q[1] += p0.y;
-    q[2] += p1.x;
-    q[3] += p1.y;
-  }
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
-  for (int o = 16; o > 0; o >>= 1)
+  double4 t = make_double4(0.0, 0.0, 0.0, 0.0);
+  if (dg.box) {
+    const int n = dg.n, nseg = (n + 31) >> 5;
+    for (int g = w; g < nseg; g += nw) {
+      const int k = 32 * g + l;
+      double4 x = make_double4(0.0, 0.0, 0.0, 0.0);
+      if (k < n) {
+        const double2 *pp = reinterpret_cast<const double2 *>(&v.pacc[dg.poff + k]);
+        const double2 p0 = __ldcg(pp), p1 = __ldcg(pp + 1);
+        x = make_double4(p0.x, p0.y, p1.x, p1.y);
+      }
 #pragma unroll
-    for (int k = 0; k < 4; k++) q[k] += __shfl_down_sync(0xffffffffu, q[k], o);
-  if (l == 0)
-    for (int k = 0; k < 4; k++) sh[k][w] = q[k];
-  __syncthreads();
+      for (int o = 1; o < 32; o <<= 1) x = xor4(x, o);
+      if (l == 0) seg[g] = x;
+    }
+    __syncthreads();
+    if (w == 0) t = total_of_segments(seg, nseg);
+  } else {
+    for (int k = threadIdx.x; k < dg.ntile_b; k += blockDim.x) {
+      const double2 *pp = reinterpret_cast<const double2 *>(&v.part_b[dg.tile0_b + k]);
+      const double2 p0 = __ldcg(pp), p1 = __ldcg(pp + 1);
+      t = add4(t, make_double4(p0.x, p0.y, p1.x, p1.y));
+    }
+    double q[4] = {t.x, t.y, t.z, t.w};
+    for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+      for (int k = 0; k < 4; k++) q[k] += __shfl_down_sync(0xffffffffu, q[k], o);
+    if (l == 0)
+      for (int k = 0; k < 4; k++) sh[k][w] = q[k];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      t = make_double4(0.0, 0.0, 0.0, 0.0);
+      for (int i = 0; i < nw; i++) t = add4(t, make_double4(sh[0][i], sh[1][i], sh[2][i], sh[3][i]));
+    }
+  }
   if (threadIdx.x == 0) {
-    double t[4] = {0.0, 0.0, 0.0, 0.0};
-    for (int i = 0; i < nw; i++)
-      for (int k = 0; k < 4; k++) t[k] += sh[k][i];
-    finalize_sums(sd, ss, dg, mode, t[0], t[1], t[2], t[3]);
+    finalize_sums(sd, ss, dg, mode, t.x, t.y, t.z, t.w);
     ss.counter_b = 0;
   }
   __syncthreads();
@@ -1919,7 +1956,7 @@ __global__ void __launch_bounds__(512) k_force_kick(View v, int mode, int tile_b
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  finalize_system(v, r, mode);
+  finalize_system(v, r, mode, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2372,7 +2409,8 @@ __device__ __forceinline__ void pair_f64(PairAcc &a, double dx, double dy, doubl
 // 207-218), forces stored, then the second half kick U2 (mode 0,
 // MDcode/time_evolve.c:558-567) or the pending thermostat scale (mode 1),
 // and the block's pe / virial / KE / active-virial partial sums
-__device__ __forceinline__ void particle_epilogue(const View &v, const SysDesc &d, const SysState &st, int i,
+template <class V>
+__device__ __forceinline__ void particle_epilogue(const V &v, const SysDesc &d, const SysState &st, int i,
                                                   int mode, const PairAcc &a, double &pe, double &vir,
                                                   double &ke, double &va) {
   const int ai = v.act[i];
@@ -2423,24 +2461,29 @@ __device__ __forceinline__ void particle_epilogue(const View &v, const SysDesc &
 // block sums stored at the block's partial slot of the system; the last block
 // of the system to finish (a counter, no waiting) finalises it
 __device__ __forceinline__ void end_force_block(const View &v, int r, int slot, int mode, double pe, double vir,
-                                                double ke, double va) {
+                                                double ke, double va, double4 *seg) {
   __shared__ double sh[32];
   __shared__ int s_last;
   const SysDesc &d = v.desc[r];
   SysState &st = v.st[r];
-  pe = block_sum_dyn(pe, sh);
-  vir = block_sum_dyn(vir, sh);
-  ke = block_sum_dyn(ke, sh);
-  va = block_sum_dyn(va, sh);
+  if (!d.box) {
+    pe = block_sum_dyn(pe, sh);
+    vir = block_sum_dyn(vir, sh);
+    ke = block_sum_dyn(ke, sh);
+    va = block_sum_dyn(va, sh);
+  } else {
+    // a whole-box system's sums are taken per particle (v.pacc) by the last block
+    __syncthreads();
+  }
   if (threadIdx.x == 0) {
-    v.part_b[d.tile0_b + slot] = make_double4(pe, vir, ke, va);
+    if (!d.box) v.part_b[d.tile0_b + slot] = make_double4(pe, vir, ke, va);
     __threadfence();
     s_last = atomicAdd(&st.counter_b, 1u) == (unsigned)(d.ntile_b - 1);
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  finalize_system(v, r, mode);
+  finalize_system(v, r, mode, seg);
 }
 
 template <int TPP, int PREC>
@@ -2629,7 +2672,7 @@ __global__ void __launch_bounds__(BLOCK_G, PREC ? ACG_FORCE_MINB32 : ACG_FORCE_M
     if (!valid || lane != 0) continue;
     particle_epilogue(v, d, st, i, mode, a, pe, vir, ke, va);
   }
-  end_force_block(v, r, tile.y, mode, pe, vir, ke, va);
+  end_force_block(v, r, tile.y, mode, pe, vir, ke, va, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2945,7 +2988,7 @@ __device__ __forceinline__ void box_list_brick(const View &v, const SysDesc &d, 
 #pragma unroll
         for (int e = 0; e < 4; e++) {
           const int qe = q + e;
-          const float4 fj = qe < q1 ? __ldg(xs + qe) : make_float4(nan, nan, nan, __int_as_float(0));
+          const float4 fj = qe < q1 ? xs[qe] : make_float4(nan, nan, nan, __int_as_float(0));
           const float ex = xi - fj.x, ey = yi - fj.y, ez = zi - fj.z;
           const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
           code[e] = __float_as_int(fj.w);
@@ -3040,7 +3083,7 @@ __device__ __forceinline__ void box_list_particle(const View &v, const SysDesc &
       bool ok = false;
       int code = 0;
       if (q < q1) {
-        const float4 fj = __ldg(xs + q);
+        const float4 fj = xs[q];
         const float ex = xi - fj.x, ey = yi - fj.y, ez = zi - fj.z;
         const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
         code = __float_as_int(fj.w);
@@ -3089,29 +3132,19 @@ __device__ __forceinline__ void box_list_particle(const View &v, const SysDesc &
   }
 }
 
-// one block per whole-box system with list sub-cells (rebuilding systems
-// only): the system in sub-cell order into xsub (reduced x, y, z as float, the
-// list code slot | type << 15) with the sub-cell starts in ssub.  A counting
-// sort in shared memory; members of a sub-cell end in slot order, so the order
-// does not depend on the atomics.
-__global__ void __launch_bounds__(BLOCK_SORT) k_sort_sub(View v) {
-  extern __shared__ int ssm[];
-  const int r = blockIdx.x;
-  if (!v.st[r].rebuild) return;
-  const SysDesc &d = v.desc[r];
-  if (!d.box || d.msub < 5) return;
-  const int n = d.n, m = d.msub, M3 = m * m * m;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int *fill = ssm;                                             // [M3]
-  int *sst = fill + M3;                                        // [M3 + 1]
-  uint16_t *key = reinterpret_cast<uint16_t *>(sst + M3 + 1);  // sub-cell of slot s
-  uint16_t *ord = key + n;                                     // slot at sorted position (unordered in a sub-cell)
-  const double4 *pp = v.pos_s + d.poff;
-  float4 *xs = v.xsub + d.poff;
+// n particles into sub-cell order by the whole block (a multiple of 32
+// threads): xs = {reduced x, y, z as float, list code slot | type << 15}, sst =
+// sub-cell starts [m^3 + 1].  pos_of(s) gives slot s's position and type; fill
+// [m^3], key [n], ord [n] are shared scratch.  A counting sort; members of a
+// sub-cell end in slot order, so the order does not depend on the atomics.
+template <class PosOf>
+__device__ __forceinline__ void sort_sub_cells(int n, int m, PosOf pos_of, int *fill, int *sst, uint16_t *key,
+                                               uint16_t *ord, float4 *xs) {
+  const int M3 = m * m * m, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int k = threadIdx.x; k < M3; k += blockDim.x) fill[k] = 0;
   __syncthreads();
   for (int s = threadIdx.x; s < n; s += blockDim.x) {
-    const double4 p = pp[s];
+    const double4 p = pos_of(s);
     const int k = subcell_of(p.x, m) + m * (subcell_of(p.y, m) + m * subcell_of(p.z, m));
     key[s] = (uint16_t)k;
     atomicAdd(&fill[k], 1);
@@ -3154,9 +3187,25 @@ __global__ void __launch_bounds__(BLOCK_SORT) k_sort_sub(View v) {
     const int q0 = sst[k], q1 = sst[k + 1];
     int rank = 0;
     for (int t = q0; t < q1; t++) rank += ord[t] < s;
-    const double4 p = pp[s];
+    const double4 p = pos_of(s);
     xs[q0 + rank] = make_float4((float)p.x, (float)p.y, (float)p.z, __int_as_float(s | ((int)p.w << 15)));
   }
+}
+
+// one block per whole-box system with list sub-cells (rebuilding systems
+// only): the system in sub-cell order into xsub with the sub-cell starts in ssub
+__global__ void __launch_bounds__(BLOCK_SORT) k_sort_sub(View v) {
+  extern __shared__ int ssm[];
+  const int r = blockIdx.x;
+  if (!v.st[r].rebuild) return;
+  const SysDesc &d = v.desc[r];
+  if (!d.box || d.msub < 5) return;
+  const int n = d.n, M3 = d.msub * d.msub * d.msub;
+  int *fill = ssm, *sst = fill + M3;
+  uint16_t *key = reinterpret_cast<uint16_t *>(sst + M3 + 1), *ord = key + n;
+  const double4 *pp = v.pos_s + d.poff;
+  sort_sub_cells(n, d.msub, [&](int s) { return pp[s]; }, fill, sst, key, ord, v.xsub + d.poff);
+  __syncthreads();
   int *gst = v.ssub + d.soff;
   for (int k = threadIdx.x; k <= M3; k += blockDim.x) gst[k] = sst[k];
 }
@@ -3306,32 +3355,31 @@ __device__ __forceinline__ void box_stage_force(const View &v, const SysDesc &d,
   }
 }
 
-// pair sums of system-local slot sl (particle i) from its list, TPP threads
-// per particle (summed across the TPP lanes on return; every thread of the
-// warp takes part)
+// pair sums of system-local slot sl (particle i, type ti) from its list of nn
+// entries (chunk c at lp[c * stride]; nn < 0: the list overflowed), TPP threads
+// per particle (summed across the TPP lanes on return; every thread of the warp
+// takes part)
 template <int TPP, int PREC>
-__device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, const unsigned char *xsm, bool valid,
-                                             int sl, int i, int lane) {
+__device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, const unsigned char *xsm,
+                                             const uint2 *lp, size_t stride, int nn, bool valid, int sl, int i,
+                                             int ti, int lane) {
   const int n = d.n;
   const int *qx = reinterpret_cast<const int *>(xsm), *qy = qx + n, *qz = qy + n;
   const double *sx = reinterpret_cast<const double *>(xsm), *sy = sx + n, *sz = sy + n;
-  const uint2 *lst = reinterpret_cast<const uint2 *>(box_list(v, d));
   const double L = d.L;
   const float scale = (float)(L * (1.0 / 4294967296.0));
-  const int nn = valid ? v.nbn[i] : 0;
   {
     PairAcc a = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid && nn >= 0) {
       const int nch = (nn + 3) >> 2;
-      const uint2 *lp = lst + sl;
-      uint2 w = lane < nch ? __ldg(lp + (size_t)lane * n) : make_uint2(0u, 0u);
+      uint2 w = lane < nch ? lp[(size_t)lane * stride] : make_uint2(0u, 0u);
       if (PREC == 1) {
         // separations in fixed-point units (L / 2^32), folded into the constants
         const unsigned xi = qx[sl], yi = qy[sl], zi = qz[sl];
-        const PairParamsF P((int)v.pos[i].w, scale);
+        const PairParamsF P(ti, scale);
         PairAccF fa = {0.f, 0.f, 0.f, 0.f, 0.f}, fb = {0.f, 0.f, 0.f, 0.f, 0.f};
         for (int c = lane; c < nch; c += TPP) {
-          const uint2 wn = c + TPP < nch ? __ldg(lp + (size_t)(c + TPP) * n) : make_uint2(0u, 0u);
+          const uint2 wn = c + TPP < nch ? lp[(size_t)(c + TPP) * stride] : make_uint2(0u, 0u);
           const int k0 = 4 * c;
 #pragma unroll
           for (int e = 0; e < 4; e++) {
@@ -3350,10 +3398,10 @@ __device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, co
         a.vir *= (double)scale;
       } else {
         const double xi = sx[sl], yi = sy[sl], zi = sz[sl];
-        const PairParamsD P((int)v.pos[i].w);
+        const PairParamsD P(ti);
         PairAcc bb = {0.0, 0.0, 0.0, 0.0, 0.0};
         for (int c = lane; c < nch; c += TPP) {
-          const uint2 wn = c + TPP < nch ? __ldg(lp + (size_t)(c + TPP) * n) : make_uint2(0u, 0u);
+          const uint2 wn = c + TPP < nch ? lp[(size_t)(c + TPP) * stride] : make_uint2(0u, 0u);
           const int k0 = 4 * c;
 #pragma unroll
           for (int e = 0; e < 4; e++) {
@@ -3375,7 +3423,6 @@ __device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, co
     } else if (valid) {
       // list overflow: all particles of the 27 neighbour images (each pair once)
       const double4 pi = v.pos[i];
-      const int ti = (int)pi.w;
       const double L2 = L * L;
       for (int k = lane; k < n; k += TPP) {
         if (k == sl) continue;
@@ -3415,13 +3462,13 @@ __global__ void __launch_bounds__(BLOCK_X, 4) k_force_box(View v, int mode) {
   const int ca = b * d.cpb, cb = min(nce, ca + d.cpb);
   const int s_lo = v.cstart[d.coff + ca], s_hi = cb < nce ? v.cstart[d.coff + cb] : n;
   __syncthreads();
-  double pe = 0.0, vir = 0.0, ke = 0.0, va = 0.0;
   const int lane = threadIdx.x % TPP, nper = blockDim.x / TPP;
   for (int t0 = s_lo; t0 < s_hi; t0 += nper) {
     const int sl = t0 + threadIdx.x / TPP;
     const bool valid = sl < s_hi;
     const int i = d.poff + (valid ? sl : s_lo);
-    PairAcc a = box_pairs<TPP, PREC>(v, d, xsm, valid, sl, i, lane);
+    PairAcc a = box_pairs<TPP, PREC>(v, d, xsm, reinterpret_cast<const uint2 *>(box_list(v, d)) + (i - d.poff), n,
+                                     valid ? v.nbn[i] : 0, valid, i - d.poff, i, (int)v.pos[i].w, lane);
     if (!valid || lane != 0) continue;
     // per-particle sums, added up in slot order by the finaliser, so the
     // system's totals do not depend on how its cells are split into blocks
@@ -3429,7 +3476,7 @@ __global__ void __launch_bounds__(BLOCK_X, 4) k_force_box(View v, int mode) {
     particle_epilogue(v, d, st, i, mode, a, pei, viri, kei, vai);
     v.pacc[i] = make_double4(pei, viri, kei, vai);
   }
-  end_force_block(v, r, b, mode, pe, vir, ke, va);
+  end_force_block(v, r, b, mode, 0.0, 0.0, 0.0, 0.0, reinterpret_cast<double4 *>(xsm));
 }
 
 // ---------------------------------------------------------------------------
