@@ -108,8 +108,9 @@ struct SysDesc {
   int shuffle, list_mode, precision, goff;  // goff: offset of the system's groups
   int tile0_a, ntile_a, box, xoff;            // kick/drift tiles; box: whole-box kernels (2..4 cells per side), xoff: first box tile
   int cpb, msub, bz, soff;                    // cpb: cells per whole-box block; msub: list sub-cells per side, bz: their list bricks' depth, soff: first sub-cell start
-  int drift_every, gsplit, gtile0, pad2;      // drift_every: remove the mean momentum after every such step (0: never);
-                                              // gsplit: force blocks per cell group, gtile0: first group force tile
+  int drift_every, gsplit, gtile0, bx_wide;      // drift_every: remove the mean momentum after every such step (0: never);
+                                              // gsplit: force blocks per cell group, gtile0: first group force tile;
+                                              // bx_wide: width of the list bricks of a system alone on a block
   double L, invL, inv_cell;  // inv_cell: cells per unit reduced length (InvCellSize)
   double T, f0, dt, half_dt, skin2, rebuild_factor, dof;
   double q[NHC_M], rq[NHC_M];  // thermostat masses and their inverses
@@ -219,10 +220,15 @@ struct View {
 };
 
 // minimum image in reduced units.  For |d| < 1.5 (all differences of wrapped
-// coordinates) d - rint(d) performs exactly the reference's operations
+// coordinates) d - round(d) performs exactly the reference's operations
 // (MDcode/cell_list+forces.c:177-182): d-1 for d > 0.5, d+1 for d < -0.5, d
-// unchanged otherwise, including d = +-0.5 (round-half-even gives 0).
-__device__ __forceinline__ double min_image(double d) { return d - rint(d); }
+// unchanged otherwise, including d = +-0.5 (round-half-even gives 0).  The
+// rounding is by adding and subtracting 1.5 2^52 (exact for |d| < 2^51): two
+// FP64 additions instead of a conversion-unit instruction.
+__device__ __forceinline__ double min_image(double d) {
+  const double m = 6755399441055744.0;
+  return __dadd_rn(d, -__dadd_rn(__dadd_rn(d, m), -m));
+}
 
 // applypbc1 (MDcode/time_evolve.c:15-26) for a displacement far below one box:
 // the while loops run at most once.  A coordinate still outside [0,1) (only

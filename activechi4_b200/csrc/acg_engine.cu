@@ -153,6 +153,8 @@ int plan(const acg_params *params, int nsys, Layout &lay, int nsm) {
         // are listed one warp each)
         const double hs = d.L / m;
         d.bz = 8.0 * hs * hs * hs * d.n / (d.L * d.L * d.L) > BRICK2_MAX ? 1 : 2;
+        // 3 x 2 x 1 bricks where those hold no more than that either
+        d.bx_wide = d.bz == 1 && 6.0 * hs * hs * hs * d.n / (d.L * d.L * d.L) <= BRICK2_MAX ? 3 : 2;
         lay.box_m3max = std::max(lay.box_m3max, m * m * m);
         d.soff = lay.nsub;
         lay.nsub += m * m * m + 1;
@@ -366,23 +368,27 @@ void plan_run(acg_engine *e, size_t smem_limit) {
     if (!run_eligible(L.desc[r])) return;
   const int C = L.nsys <= 7 ? 16 : (L.nsys <= 15 ? 8 : (L.nsys <= 33 ? 4 : (L.nsys <= 74 ? 2 : 1)));
   const int prec = L.desc[0].precision;
+  // state in shared memory where it fits; threads per block: 512 (FP64 pair
+  // terms take about 120 registers a thread), or 1024 for FP32 systems with
+  // more slots per block than that
   for (int resident = 1; resident >= 0; resident--) {
-    size_t least = 0, want = 0;
     int nloc = 0;
-    for (int r = 0; r < L.nsys; r++) {
-      const SysDesc &d = L.desc[r];
-      const RunPlan p = run_plan(d.n, d.ncell, d.msub, prec, C, resident);
+    for (const SysDesc &d : L.desc) nloc = std::max(nloc, 32 * (((d.n + 31) / 32 + C - 1) / C));
+    const int nt = prec && !resident && nloc * 2 > 512 ? 1024 : 512;
+    size_t least = 0, want = 0;
+    for (const SysDesc &d : L.desc) {
+      const RunPlan p = run_plan(d.n, d.ncell, d.msub, prec, C, resident, nt / 32);
       least = std::max(least, p.least());
-      // and the lists of the block's slots, about 120 entries of two bytes each
+      // and the lists of the block's slots, about 120 entries of two bytes each,
+      // and list buffers for all warps
       want = std::max(want, p.pool + p.stage_bytes + 256 * (size_t)p.nloc + p.perm_bytes);
-      nloc = std::max(nloc, p.nloc);
+      want = std::max(want, p.pool + p.lists_at + sizeof(BrickScratch) * (nt / 32) + p.perm_bytes);
     }
     if (least > smem_limit) continue;
     e->run_c = C;
+    e->run_nt = nt;
     e->run_resident = resident;
     e->run_smem = std::min(smem_limit, std::max(least, want));
-    // FP64 pair terms take about 120 registers a thread
-    e->run_nt = prec && !resident && nloc * 2 > 512 ? 1024 : 512;
     return;
   }
 }

@@ -1715,15 +1715,14 @@ __global__ void k_lattice(View v, int r, int troot) {
 }
 
 // 1/x for x in the pair range (0.3 < x < 7): the hardware estimate
-// (rcp.approx.ftz.f64) refined by two Newton-Raphson steps y += y (1 - x y),
-// each squaring the relative error, to within an ulp of the rounded quotient
+// (rcp.approx.ftz.f64, relative error e below 2^-20) refined by one step of
+// Halley's third-order iteration, y (1 + e + e^2) with e = 1 - x y: the error
+// becomes e^3, below the rounding, in three operations
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
 // 1/x in FP32 from the hardware estimate (a Newton step on it changed the
@@ -1738,41 +1737,48 @@ struct PairAccF {
   float fx, fy, fz, pe, vir;
 };
 
-// the sums of one list chunk (at most two FP32 terms in each of fa, fb) moved
-// into the FP64 sums: the per-particle force is a sum of large terms of both
-// signs, whose FP32 rounding would otherwise grow with the list; and the FP64
-// sum of these chunk values is exact in practice, so it does not depend on how
-// the chunks are split over threads
-__device__ __forceinline__ void flush_chunk(PairAccF &fa, PairAccF &fb, PairAcc &a) {
-  a.fx += (double)(fa.fx + fb.fx);
-  a.fy += (double)(fa.fy + fb.fy);
-  a.fz += (double)(fa.fz + fb.fz);
-  a.pe += (double)(fa.pe + fb.pe);
-  a.vir += (double)(fa.vir + fb.vir);
-  fa = PairAccF{0.f, 0.f, 0.f, 0.f, 0.f};
-  fb = PairAccF{0.f, 0.f, 0.f, 0.f, 0.f};
+// the FP32 sums of one list chunk (at most four terms) moved into the FP64
+// sums: the per-particle force is a sum of large terms of both signs, whose
+// FP32 rounding would otherwise grow with the list; and the FP64 sum of these
+// chunk values is exact in practice, so it does not depend on how the chunks
+// are split over threads
+__device__ __forceinline__ void flush_chunk(PairAccF &f, PairAcc &a) {
+  a.fx += (double)f.fx;
+  a.fy += (double)f.fy;
+  a.fz += (double)f.fz;
+  a.pe += (double)f.pe;
+  a.vir += (double)f.vir;
+  f = PairAccF{0.f, 0.f, 0.f, 0.f, 0.f};
 }
 
-// FP32 pair constants of particle i against a partner of type 0 and of type 1:
-// 1/sigma^2, 4 eps and 8 eps/sigma^2 (MDcode/cell_list+forces.c:19-20)
+// 1/sigma^2 and 4 eps of a pair by its type sum (MDcode/cell_list+forces.c:19-20)
+__device__ __forceinline__ double ka_is2(int tp) { return tp == 0 ? 1.0 : (tp == 1 ? 1.5625 : 1.0 / (0.88 * 0.88)); }
+__device__ __forceinline__ double ka_e4(int tp) { return tp == 0 ? 4.0 : (tp == 1 ? 6.0 : 2.0); }
+
+// The pair terms below take separations counted in units u of length (u^2 is
+// folded into 1/sigma^2) and add up pe, h d and h d^2 with
+// h = 4 eps u^2/sigma^2 (s6 (6 s6 - 3) s2 - C2), half of the radial force factor
+// times u^2: in absolute units the force is 2/u and the virial 2 times the sums
+// (pair_scale).  Everything is evaluated for every list entry and masked by a
+// zero 4 eps beyond the cut or the list's end (no divergent branch: the entries
+// of a chunk interleave, and each sum gains exactly nothing; the entries that
+// pad a list repeat its last one or lie far away, so every term is finite).
+__device__ __forceinline__ void pair_scale(PairAcc &a, double u) {
+  const double c = 2.0 / u;
+  a.fx *= c;
+  a.fy *= c;
+  a.fz *= c;
+  a.vir *= 2.0;
+}
+
+// FP32 pair constants of particle i against a partner of type 0 and of type 1
 struct PairParamsF {
-  float is2[2], e4[2], ge[2];
-  __device__ __forceinline__ explicit PairParamsF(int ti) {
+  float is2[2], e4[2];
+  __device__ __forceinline__ PairParamsF(int ti, double u) {
 #pragma unroll
     for (int tj = 0; tj < 2; tj++) {
-      const int tp = ti + tj;
-      is2[tj] = tp == 0 ? 1.0f : (tp == 1 ? 1.5625f : (float)(1.0 / (0.88 * 0.88)));
-      e4[tj] = tp == 0 ? 4.0f : (tp == 1 ? 6.0f : 2.0f);
-      ge[tj] = 2.0f * e4[tj] * is2[tj];
-    }
-  }
-  // for separations counted in units of u: 1/sigma^2 u^2 and 8 eps/sigma^2 u,
-  // so forces come out in absolute units and the virial in units of 1/u
-  __device__ __forceinline__ PairParamsF(int ti, float u) : PairParamsF(ti) {
-#pragma unroll
-    for (int tj = 0; tj < 2; tj++) {
-      is2[tj] *= u * u;
-      ge[tj] *= u;
+      is2[tj] = (float)(ka_is2(ti + tj) * (u * u));
+      e4[tj] = (float)ka_e4(ti + tj);
     }
   }
 };
@@ -1780,22 +1786,51 @@ struct PairParamsF {
 // FP32 pair term: U = 4 eps (s^12 - s^6) + C0 + C2 (r/sigma)^2 and its radial
 // force factor, written as s6 (s6 - 1) and s6 (6 s6 - 3) s2
 __device__ __forceinline__ void pair_f32(PairAccF &a, float dx, float dy, float dz, const PairParamsF &P,
-                                         bool tj) {
+                                         bool tj, bool valid) {
   const float is2 = tj ? P.is2[1] : P.is2[0];
   const float dr2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
   const float rs2 = dr2 * is2;
-  // evaluated for every entry and masked (no divergent branch): beyond the cut
-  // the factors are zero and each sum gains exactly nothing
-  const bool in = rs2 < (float)KA_RC2;
-  const float e4 = in ? (tj ? P.e4[1] : P.e4[0]) : 0.0f, ge = in ? (tj ? P.ge[1] : P.ge[0]) : 0.0f;
+  const bool in = rs2 < (float)KA_RC2 && valid;
+  const float e4 = in ? (tj ? P.e4[1] : P.e4[0]) : 0.0f;
   const float s2 = rcp_approx(rs2);
   const float s6 = s2 * s2 * s2;
   a.pe = fmaf(e4, fmaf(s6, s6, -s6) + fmaf((float)KA_C2, rs2, (float)KA_C0), a.pe);
-  const float g = ge * fmaf(s6 * fmaf(6.0f, s6, -3.0f), s2, -(float)KA_C2);
+  const float g = (e4 * is2) * fmaf(s6 * fmaf(6.0f, s6, -3.0f), s2, -(float)KA_C2);
   a.fx = fmaf(g, dx, a.fx);
   a.fy = fmaf(g, dy, a.fy);
   a.fz = fmaf(g, dz, a.fz);
   a.vir = fmaf(g, dr2, a.vir);
+}
+
+// FP64 pair constants; 4 eps by its high word (4, 6 and 2 have an empty low one)
+struct PairParamsD {
+  double is2[2];
+  int e4hi[2];
+  __device__ __forceinline__ PairParamsD(int ti, double u) {
+#pragma unroll
+    for (int tj = 0; tj < 2; tj++) {
+      is2[tj] = ka_is2(ti + tj) * (u * u);
+      e4hi[tj] = __double2hiint(ka_e4(ti + tj));
+    }
+  }
+};
+
+// FP64 pair term (MDcode/cell_list+forces.c:174-203), in fused multiply-adds
+__device__ __forceinline__ void pair_f64(PairAcc &a, double dx, double dy, double dz, const PairParamsD &P,
+                                         bool tj, bool valid) {
+  const double is2 = tj ? P.is2[1] : P.is2[0];
+  const double dr2 = fma(dx, dx, fma(dy, dy, dz * dz));
+  const double rs2 = dr2 * is2;
+  const bool in = rs2 < KA_RC2 && valid;
+  const double e4 = __hiloint2double(in ? (tj ? P.e4hi[1] : P.e4hi[0]) : 0, 0);
+  const double s2 = rcp_nr(rs2);
+  const double s6 = s2 * s2 * s2;
+  a.pe = fma(e4, fma(s6, s6, -s6) + fma(KA_C2, rs2, KA_C0), a.pe);
+  const double g = (e4 * is2) * fma(s6 * fma(6.0, s6, -3.0), s2, -KA_C2);
+  a.fx = fma(g, dx, a.fx);
+  a.fy = fma(g, dy, a.fy);
+  a.fz = fma(g, dz, a.fz);
+  a.vir = fma(g, dr2, a.vir);
 }
 
 // stage 2: forces + second kick.  mode 0 = step; 1 = prime (forces at the
@@ -1821,11 +1856,13 @@ __global__ void __launch_bounds__(512) k_force_kick(View v, int mode, int tile_b
   if (valid) {
     const double4 pi = v.pos[i];
     const int ti = (int)pi.w;
-    const PairParamsF PF(ti);
+    const PairParamsF PF(ti, 1.0);
+    const PairParamsD PD(ti, L);
     const int nn = v.nbn[i];
     if (nn >= 0) {
       // four list entries per lane per iteration (one 16-byte load; rows are
-      // 16-byte aligned and padded to maxnb, entries past nn are not used)
+      // 16-byte aligned and padded to maxnb; an entry past nn takes the
+      // chunk's first particle and is masked)
       const int4 *row4 = reinterpret_cast<const int4 *>(v.nbl + (size_t)i * v.maxnb);
       const int nb4 = (nn + 3) >> 2;
       // each chunk's slots are loaded one iteration ahead, so the positions it
@@ -1834,37 +1871,26 @@ __global__ void __launch_bounds__(512) k_force_kick(View v, int mode, int tile_b
       for (int b = lane; b < nb4; b += TPP) {
         const int4 jj = jn;
         if (b + TPP < nb4) jn = __ldg(row4 + b + TPP);
-        const int k0 = 4 * b;
-        const bool v1 = k0 + 1 < nn, v2 = k0 + 2 < nn, v3 = k0 + 3 < nn;
-        const double4 p0 = v.pos[jj.x];
-        const double4 p1 = v1 ? v.pos[jj.y] : pi;
-        const double4 p2 = v2 ? v.pos[jj.z] : pi;
-        const double4 p3 = v3 ? v.pos[jj.w] : pi;
-        if (PREC == 0) {
-          pair_fp64(a, pi, ti, p0, L, L2);
-          if (v1) pair_fp64(a, pi, ti, p1, L, L2);
-          if (v2) pair_fp64(a, pi, ti, p2, L, L2);
-          if (v3) pair_fp64(a, pi, ti, p3, L, L2);
-        } else {
-          // separations from the FP64 minimum image, the pair terms in FP32
-          // summed per chunk of four and moved into the FP64 sums (as the
-          // cell-group and whole-box kernels do); an unused entry (past nn)
-          // is the particle itself at separation zero, masked by the cut test
-          const float Lf = (float)L;
-          PairAccF fa = {0.f, 0.f, 0.f, 0.f, 0.f}, fb = {0.f, 0.f, 0.f, 0.f, 0.f};
-          const double4 pj[4] = {p0, p1, p2, p3};
+        const int left = nn - 4 * b;
+        const double4 pj[4] = {v.pos[jj.x], v.pos[left > 1 ? jj.y : jj.x], v.pos[left > 2 ? jj.z : jj.x],
+                               v.pos[left > 3 ? jj.w : jj.x]};
+        // separations from the FP64 minimum image; FP32 pair terms are summed
+        // per chunk of four and moved into the FP64 sums (as the cell-group
+        // and whole-box kernels do)
+        PairAccF f = {0.f, 0.f, 0.f, 0.f, 0.f};
+        const float Lf = (float)L;
 #pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const float dx = (float)min_image(pi.x - pj[e].x) * Lf;
-            const float dy = (float)min_image(pi.y - pj[e].y) * Lf;
-            const float dz = (float)min_image(pi.z - pj[e].z) * Lf;
-            const float dr2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
-            // separation zero (the particle itself in an unused entry) gains nothing
-            if (dr2 > 0.0f) pair_f32(e & 1 ? fb : fa, dx, dy, dz, PF, (int)pj[e].w != 0);
-          }
-          flush_chunk(fa, fb, a);
+        for (int e = 0; e < 4; e++) {
+          const double dx = min_image(pi.x - pj[e].x), dy = min_image(pi.y - pj[e].y), dz = min_image(pi.z - pj[e].z);
+          const bool tj = __double2hiint(pj[e].w) != 0;
+          if (PREC == 0)
+            pair_f64(a, dx, dy, dz, PD, tj, e < left);
+          else
+            pair_f32(f, (float)dx * Lf, (float)dy * Lf, (float)dz * Lf, PF, tj, e < left);
         }
+        if (PREC == 1) flush_chunk(f, a);
       }
+      pair_scale(a, PREC == 0 ? L : 1.0);
     } else {
       // neighbour-list overflow: scan the cells around the cell of the last
       // rebuild (every pair within the cut is there since displacements stay
@@ -2354,46 +2380,6 @@ __global__ void __launch_bounds__(BLOCK_G) k_build_list_groups(View v) {
   }
 }
 
-// FP64 pair constants of particle i against a partner of type 0 and of type 1:
-// 1/sigma^2, 4 eps and 8 eps/sigma^2 (MDcode/cell_list+forces.c:19-20)
-struct PairParamsD {
-  double is2[2], e4[2], ge[2];
-  __device__ __forceinline__ explicit PairParamsD(int ti) {
-#pragma unroll
-    for (int tj = 0; tj < 2; tj++) {
-      const int tp = ti + tj;
-      is2[tj] = tp == 0 ? 1.0 : (tp == 1 ? 1.5625 : 1.0 / (0.88 * 0.88));
-      e4[tj] = tp == 0 ? 4.0 : (tp == 1 ? 6.0 : 2.0);
-      ge[tj] = 2.0 * e4[tj] * is2[tj];
-    }
-  }
-};
-
-// FP64 pair term on a separation already in the minimum image (absolute
-// units): U = 4 eps (s^12 - s^6) + C0 + C2 (r/sigma)^2 and the radial force
-// factor 8 eps/sigma^2 (s6 (6 s6 - 3) s2 - C2), s2 = sigma^2/r^2
-// (MDcode/cell_list+forces.c:174-203), written in fused multiply-adds
-__device__ __forceinline__ void pair_f64(PairAcc &a, double dx, double dy, double dz, const PairParamsD &P,
-                                         bool tj) {
-  const double is2 = tj ? P.is2[1] : P.is2[0];
-  const double dr2 = fma(dx, dx, fma(dy, dy, dz * dz));
-  const double rs2 = dr2 * is2;
-  // evaluated for every entry and masked, as the FP32 term: beyond the cut
-  // (s2 <= 0.16, every product finite) the factors are zero and each sum
-  // gains an exact zero, so the sums are those of a branch on the cut; with
-  // no branch the four pairs of a list chunk interleave
-  const bool in = rs2 < KA_RC2;
-  const double e4 = in ? (tj ? P.e4[1] : P.e4[0]) : 0.0, ge = in ? (tj ? P.ge[1] : P.ge[0]) : 0.0;
-  const double s2 = rcp_nr(rs2);
-  const double s6 = s2 * s2 * s2;
-  a.pe = fma(e4, fma(s6, s6, -s6) + fma(KA_C2, rs2, KA_C0), a.pe);
-  const double g = ge * fma(s6 * fma(6.0, s6, -3.0), s2, -KA_C2);
-  a.fx = fma(g, dx, a.fx);
-  a.fy = fma(g, dy, a.fy);
-  a.fz = fma(g, dz, a.fz);
-  a.vir = fma(g, dr2, a.vir);
-}
-
 // launch-bounds occupancy targets of the cell-group force kernel (blocks per
 // SM).  FP64: 2, no spills (the masked pair term interleaves the four pairs of
 // a chunk; at 4 blocks, 64 registers, it spilled: N = 2.56e5 force 143 -> 129
@@ -2581,10 +2567,10 @@ __global__ void __launch_bounds__(BLOCK_G, PREC ? ACG_FORCE_MINB32 : ACG_FORCE_M
     if (PREC == 1 && valid && staged && nn >= 0) {
       const float4 hi = shi[qs];
       const float2 li = slo[qs];
-      const PairParamsF P(ti);
+      const PairParamsF P(ti, 1.0);
       const int nch = (nn + 3) >> 2;
       const uint2 *lp = reinterpret_cast<const uint2 *>(lst) + t;
-      PairAccF fa = {0.f, 0.f, 0.f, 0.f, 0.f}, fb = {0.f, 0.f, 0.f, 0.f, 0.f};
+      PairAccF f = {0.f, 0.f, 0.f, 0.f, 0.f};
       uint2 w = lane < nch ? __ldg(lp + (size_t)lane * M) : make_uint2(0u, 0u);
       for (int c = lane; c < nch; c += TPP) {
         const uint2 wn = c + TPP < nch ? __ldg(lp + (size_t)(c + TPP) * M) : make_uint2(0u, 0u);
@@ -2597,14 +2583,15 @@ __global__ void __launch_bounds__(BLOCK_G, PREC ? ACG_FORCE_MINB32 : ACG_FORCE_M
           const float dx = (hi.x - hj.x) + (hi.w - hj.w);
           const float dy = (hi.y - hj.y) + (li.x - lj.x);
           const float dz = (hi.z - hj.z) + (li.y - lj.y);
-          pair_f32(e & 1 ? fb : fa, dx, dy, dz, P, code >> 15);
+          pair_f32(f, dx, dy, dz, P, code >> 15, true);
         }
-        flush_chunk(fa, fb, a);
+        flush_chunk(f, a);
         w = wn;
       }
+      pair_scale(a, 1.0);
     } else if (PREC == 0 && valid && staged && nn >= 0) {
       const double xi = sx[qs], yi = sy[qs], zi = sz[qs];
-      const PairParamsD P(ti);
+      const PairParamsD P(ti, 1.0);
       const int nch = (nn + 3) >> 2;
       const uint2 *lp = reinterpret_cast<const uint2 *>(lst) + t;
       // list chunks are loaded two iterations ahead (an L2 round trip is
@@ -2618,19 +2605,19 @@ __global__ void __launch_bounds__(BLOCK_G, PREC ? ACG_FORCE_MINB32 : ACG_FORCE_M
         const int e0 = w.x & 0xffff, e1 = w.x >> 16, e2 = w.y & 0xffff, e3 = w.y >> 16;
         {
           const int q = e0 & 0x7fff;
-          pair_f64(a, xi - sx[q], yi - sy[q], zi - sz[q], P, e0 >> 15);
+          pair_f64(a, xi - sx[q], yi - sy[q], zi - sz[q], P, e0 >> 15, true);
         }
         {
           const int q = e1 & 0x7fff;
-          pair_f64(b, xi - sx[q], yi - sy[q], zi - sz[q], P, e1 >> 15);
+          pair_f64(b, xi - sx[q], yi - sy[q], zi - sz[q], P, e1 >> 15, true);
         }
         {
           const int q = e2 & 0x7fff;
-          pair_f64(a, xi - sx[q], yi - sy[q], zi - sz[q], P, e2 >> 15);
+          pair_f64(a, xi - sx[q], yi - sy[q], zi - sz[q], P, e2 >> 15, true);
         }
         {
           const int q = e3 & 0x7fff;
-          pair_f64(b, xi - sx[q], yi - sy[q], zi - sz[q], P, e3 >> 15);
+          pair_f64(b, xi - sx[q], yi - sy[q], zi - sz[q], P, e3 >> 15, true);
         }
         w = wn;
         wn = wnn;
@@ -2640,6 +2627,7 @@ __global__ void __launch_bounds__(BLOCK_G, PREC ? ACG_FORCE_MINB32 : ACG_FORCE_M
       a.fz += b.fz;
       a.pe += b.pe;
       a.vir += b.vir;
+      pair_scale(a, 1.0);
     } else if (valid) {
       // list overflow or oversized union: scan the neighbour cells directly
       const int nc = d.nc, c = v.cellof[i];
@@ -2722,102 +2710,6 @@ __device__ __forceinline__ void box_cells(const View &v, const SysDesc &d, int *
     }
   }
   __syncthreads();
-}
-
-// lists of the particles of cell c of a whole box (one warp; lanes are the
-// particles of the cell, in rounds of 32) against the staged system: the 27
-// neighbour cells with their periodic image shifts (at 2 cells per side a cell
-// appears under two shifts, of which at most one can be in range since L > 2 x
-// the list cut), candidates in slot order within each cell
-__device__ __forceinline__ void box_list_cell(const View &v, const SysDesc &d, int r, const float4 *xstg,
-                                              const int *cst, const int *pre4, int c, int lane, int round0,
-                                              int rstep) {
-  const int nc = d.nc, n = d.n;
-  const double iL2 = 1.0 / (d.L * d.L);
-  float lc[3];
-  for (int k = 0; k < 3; k++) lc[k] = (float)(lcut2_of(d, k) * iL2 * (1.0 + 1e-5));
-  const bool one_cut = lc[0] == lc[1] && lc[1] == lc[2];
-  uint2 *lst = reinterpret_cast<uint2 *>(box_list(v, d));
-  const int maxnb = v.maxnb;
-  {
-
-    const int cx = c % nc, cy = (c / nc) % nc, cz = c / (nc * nc);
-    const int m = cst[c + 1] - cst[c];
-    for (int w0 = 32 * round0; w0 < m; w0 += 32 * rstep) {
-      const int w = w0 + lane;
-      const bool valid = w < m;
-      const int sl = cst[c] + w, ps = pre4[c] + w;
-      // a lane past the cell's particles gets NaN coordinates: it passes no test
-      const float nan = __int_as_float(0x7fc00000);
-      const float4 fi = valid ? xstg[ps] : make_float4(nan, nan, nan, __int_as_float(0));
-      const int ti = __float_as_int(fi.w) >> 15;
-      const float c0 = ti == 0 ? lc[0] : lc[1], c1 = ti == 0 ? lc[1] : lc[2];
-      ListWriter lw;
-      if (nc == 2) {
-        // two cells per side: every cell neighbours every other under two
-        // images, so test each particle once with the minimum image instead
-        // of 27 images of 8 cells
-        const int q1 = pre4[d.ncell];
-        for (int q = 0; q < q1; q += 4) {
-          int code[4];
-          bool ok[4];
-#pragma unroll
-          for (int e = 0; e < 4; e++) {
-            const float4 fj = xstg[q + e];
-            float ex = fi.x - fj.x, ey = fi.y - fj.y, ez = fi.z - fj.z;
-            ex -= rintf(ex);
-            ey -= rintf(ey);
-            ez -= rintf(ez);
-            const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-            code[e] = __float_as_int(fj.w);
-            const float cut = one_cut ? c0 : ((code[e] >> 15) ? c1 : c0);
-            ok[e] = valid && r2 < cut && q + e != ps;
-          }
-#pragma unroll
-          for (int e = 0; e < 4; e++)
-            if (ok[e]) lw.add((unsigned)code[e] & 0xffffu, lst, n, sl, maxnb);
-        }
-      }
-      for (int dz = -1; dz <= 1 && nc > 2; dz++)
-        for (int dy = -1; dy <= 1; dy++)
-          for (int dx = -1; dx <= 1; dx++) {
-            const int ax = cx + dx, ay = cy + dy, az = cz + dz;
-            const int sx = ax < 0 ? -1 : (ax >= nc ? 1 : 0), sy = ay < 0 ? -1 : (ay >= nc ? 1 : 0),
-                      sz = az < 0 ? -1 : (az >= nc ? 1 : 0);
-            const int c2 = (ax - sx * nc) + (ay - sy * nc) * nc + (az - sz * nc) * nc * nc;
-            // candidate image x_j + s: compare x_i - s with x_j
-            const float xi = fi.x - (float)sx, yi = fi.y - (float)sy, zi = fi.z - (float)sz;
-            const int q1 = pre4[c2 + 1];
-            for (int q = pre4[c2]; q < q1; q += 4) {
-              int code[4];
-              bool ok[4];
-#pragma unroll
-              for (int e = 0; e < 4; e++) {
-                const float4 fj = xstg[q + e];
-                const float ex = xi - fj.x, ey = yi - fj.y, ez = zi - fj.z;
-                const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-                code[e] = __float_as_int(fj.w);
-                const float cut = one_cut ? c0 : ((code[e] >> 15) ? c1 : c0);
-                ok[e] = valid && r2 < cut && q + e != ps;
-              }
-#pragma unroll
-              for (int e = 0; e < 4; e++)
-                if (ok[e]) lw.add((unsigned)code[e] & 0xffffu, lst, n, sl, maxnb);
-            }
-          }
-      if (valid) {
-        lw.finish(lst, n, sl, maxnb);
-        const int nn = lw.n;
-        const int i = d.poff + sl;
-        if (nn > maxnb) {
-          v.nbn[i] = -1;
-          atomicAdd(&v.st[r].overflow, 1);
-        } else {
-          v.nbn[i] = nn;
-        }
-      }
-    }
-  }
 }
 
 // the system in cell order (after the permutation) as float4 {reduced x, y, z,
@@ -2907,6 +2799,12 @@ __device__ __forceinline__ void box_list_group(const View &v, const SysDesc &d, 
           scan(pre4[c2], pre4[c2 + 1], fi.x - (float)sx, fi.y - (float)sy, fi.z - (float)sz, false);
         }
   }
+  // the rest of the last chunk repeats the last entry
+  __syncwarp();
+  if (valid && (cnt & 3) && sub >= (cnt & 3) && cnt <= maxnb) {
+    const size_t at = ((size_t)(cnt >> 2) * n + sl) * 4;
+    lst[at + sub] = lst[at + (cnt & 3) - 1];
+  }
   if (valid && sub == 0) {
     const int i = d.poff + sl;
     if (cnt > maxnb) {
@@ -2930,26 +2828,51 @@ __device__ __forceinline__ void box_list_group(const View &v, const SysDesc &d, 
 // particles) or bricks of 2 x 2 x d.bz sub-cells, one lane per particle.
 __device__ __forceinline__ int subcell_of(double x, int m) { return min(max((int)(x * (double)m), 0), m - 1); }
 
-// lists of the particles of brick B (2 x 2 x d.bz sub-cells), one lane per
-// particle in rounds of 32: every lane tests the same candidate (a broadcast
-// load of the sorted system) from the union of the brick's sub-cells' 5 x 5 x 5
-// neighbourhoods,
-// rows of up to 6 sub-cells contiguous in sub-cell order.  Where the union is
-// wider than the box (5 sub-cells per side) a sub-cell comes under two image
-// shifts, of which at most one can be in range (L > 2 x the list cut).
+// the cuts of a whole-box list for a partner of type 0 / 1 (reduced units,
+// widened by 1e-5), the same expression in every list builder
+__device__ __forceinline__ void box_cuts(const SysDesc &d, int ti, float &c0, float &c1) {
+  const double iL2 = 1.0 / (d.L * d.L);
+  c0 = (float)(lcut2_of(d, ti) * iL2 * (1.0 + 1e-5));
+  c1 = (float)(lcut2_of(d, ti + 1) * iL2 * (1.0 + 1e-5));
+}
+
 __device__ __forceinline__ void box_list_particle(const View &v, const SysDesc &d, int r, const float4 *xs,
                                                   const int *sst, int ps, int lane);
 
+// lists of the particles of brick B (bx x 2 x bz sub-cells), one lane per
+// particle: every lane tests the same candidate (a broadcast load) from the
+// union of the brick's sub-cells' 5 x 5 x 5 neighbourhoods, rows of up to 7
+// sub-cells contiguous in sub-cell order.  Where the union is wider than the
+// box (5 sub-cells per side) a sub-cell comes under two image shifts, of which at
+// most one can be in range (L > 2 x the list cut).
+//
+// What bounds it: instruction issue, 700 to 900 candidates a sweep.  The warp
+// first writes down the union's runs; its lanes then fetch 32 candidates at a
+// time, whatever runs they lie in, with their image shift into shared memory, so
+// the tests run without run ends, shifts or loop heads in between.  An accepted
+// candidate goes to the lane's column of codes by a predicated store and a
+// pointer step, not a branch (with 32 lanes nearly every candidate is accepted by
+// one of them, so all would pay for the append); full chunks of four move to
+// the list after every 32 (with 64 at a time the buffers of fewer warps fit:
+// the 256-replica step 245 against 250 us).  Appending in registers behind a
+// branch took about 26 instructions a candidate in all, this 19: a rebuild of
+// N = 3997 on one SM 1.9e6 -> 1.4e6 cycles.
+constexpr int BRICK_ROWS = 36;  // (z, y) rows of a union at most (2 x 2 x 2 bricks)
+constexpr int BRICK_BATCH = 32;
+struct BrickScratch {           // one warp's shared memory
+  float4 cand[BRICK_BATCH];
+  uint16_t col[BRICK_BATCH + 4][32];  // a batch's entries and three left over per lane
+  uint16_t start[3 * BRICK_ROWS], first[3 * BRICK_ROWS + 4];  // runs: start in sub-cell order, candidates before
+  signed char sy[BRICK_ROWS], sz[BRICK_ROWS];                 // image of each row
+};
+static_assert(sizeof(BrickScratch) % 16 == 0, "arrays of it keep float4 aligned");
 __device__ __forceinline__ void box_list_brick(const View &v, const SysDesc &d, int r, const float4 *xs,
-                                               const int *sst, int B, int lane) {
-  const int m = d.msub, bz = d.bz, n = d.n;
-  const int nbx = (m + 1) >> 1;
-  const int Bx = B % nbx, By = (B / nbx) % nbx, Bz = B / (nbx * nbx);
-  const int x0 = 2 * Bx, x1 = min(x0 + 2, m), y0 = 2 * By, y1 = min(y0 + 2, m), z0 = bz * Bz,
+                                               const int *sst, int B, int bx, int bz, int lane, BrickScratch &S) {
+  const int m = d.msub, n = d.n;
+  const int nbx = (m + bx - 1) / bx, nby = (m + 1) >> 1;
+  const int Bx = B % nbx, By = (B / nbx) % nby, Bz = B / (nbx * nby);
+  const int x0 = bx * Bx, x1 = min(x0 + bx, m), y0 = 2 * By, y1 = min(y0 + 2, m), z0 = bz * Bz,
             z1 = min(z0 + bz, m);
-  const double iL2 = 1.0 / (d.L * d.L);
-  float lc[3];
-  for (int k = 0; k < 3; k++) lc[k] = (float)(lcut2_of(d, k) * iL2 * (1.0 + 1e-5));
   uint2 *lst = reinterpret_cast<uint2 *>(box_list(v, d));
   const int maxnb = v.maxnb;
   const float nan = __int_as_float(0x7fc00000);
@@ -2959,78 +2882,144 @@ __device__ __forceinline__ void box_list_brick(const View &v, const SysDesc &d, 
       const int row = m * (y + m * z);
       total += sst[row + x1] - sst[row + x0];
     }
+  // the union's runs in (z, y) order, three per row in increasing unwrapped x:
+  // image to the left, the box itself, image to the right (some empty)
+  const int ny = y1 - y0 + 4, nrow = (z1 - z0 + 4) * ny;
+  int Q = 0;
+  for (int r0 = 0; r0 < nrow; r0 += 32) {
+    const int rr = r0 + lane;
+    int len[3] = {0, 0, 0};
+    if (rr < nrow) {
+      const int zz = z0 - 2 + rr / ny, yy = y0 - 2 + rr % ny;
+      const int sz = zz < 0 ? -1 : (zz >= m ? 1 : 0), sy = yy < 0 ? -1 : (yy >= m ? 1 : 0);
+      const int row = m * ((yy - sy * m) + m * (zz - sz * m));
+      const int xa = x0 - 2, xb = x1 + 2;
+      const int q[3] = {sst[row + m + min(xa, 0)], sst[row + max(xa, 0)], sst[row]};
+      len[0] = sst[row + m] - q[0];
+      len[1] = sst[row + min(xb, m)] - q[1];
+      len[2] = sst[row + max(xb - m, 0)] - q[2];
+      S.sy[rr] = (signed char)sy;
+      S.sz[rr] = (signed char)sz;
+      for (int k = 0; k < 3; k++) S.start[3 * rr + k] = (uint16_t)q[k];
+    }
+    const int mine = len[0] + len[1] + len[2];
+    int x = mine;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int y = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += y;
+    }
+    if (rr < nrow) {
+      S.first[3 * rr] = (uint16_t)(Q + x - mine);
+      S.first[3 * rr + 1] = (uint16_t)(Q + x - mine + len[0]);
+      S.first[3 * rr + 2] = (uint16_t)(Q + x - len[2]);
+    }
+    Q += __shfl_sync(0xffffffffu, x, 31);
+  }
+  if (lane == 0) S.first[3 * nrow] = 0xffffu;
   // the brick's first 32 particles, one lane each; the others (a dense
   // brick) one warp each below, so the warp does not sweep the brick's
   // neighbourhood a second time for a few lanes
-  {
-    // this lane's particle: entry k of the brick's runs (z, y) of x0..x1-1
-    int k = lane, ps = -1;
-    for (int z = z0; z < z1; z++)
-      for (int y = y0; y < y1; y++) {
-        const int row = m * (y + m * z);
-        const int q0 = sst[row + x0], len = sst[row + x1] - q0;
-        if (ps < 0) {
-          if (k < len) ps = q0 + k;
-          else k -= len;
-        }
-      }
-    const bool valid = ps >= 0;
-    // a lane past the brick's particles gets NaN coordinates: it passes no test
-    const float4 fi = valid ? xs[ps] : make_float4(nan, nan, nan, __int_as_float(0));
-    const int codei = __float_as_int(fi.w);
-    const int sl = codei & 0x7fff, ti = codei >> 15;
-    const float c0 = ti == 0 ? lc[0] : lc[1], c1 = ti == 0 ? lc[1] : lc[2];
-    ListWriter lw;
-    auto run = [&](int q0, int q1, float xi, float yi, float zi) {
-      for (int q = q0; q < q1; q += 4) {
-        int code[4];
-        bool ok[4];
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-          const int qe = q + e;
-          const float4 fj = qe < q1 ? xs[qe] : make_float4(nan, nan, nan, __int_as_float(0));
-          const float ex = xi - fj.x, ey = yi - fj.y, ez = zi - fj.z;
-          const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-          code[e] = __float_as_int(fj.w);
-          ok[e] = r2 < ((code[e] >> 15) ? c1 : c0) && qe != ps;
-        }
-#pragma unroll
-        for (int e = 0; e < 4; e++)
-          if (ok[e]) lw.add((unsigned)code[e] & 0xffffu, lst, n, sl, maxnb);
-      }
-    };
-    for (int zz = z0 - 2; zz < z1 + 2; zz++) {
-      const int sz = zz < 0 ? -1 : (zz >= m ? 1 : 0), az = zz - sz * m;
-      for (int yy = y0 - 2; yy < y1 + 2; yy++) {
-        const int sy = yy < 0 ? -1 : (yy >= m ? 1 : 0), ay = yy - sy * m;
-        const int row = m * (ay + m * az);
-        // candidate image x_j + s: compare x_i - s with x_j
-        const float yi = fi.y - (float)sy, zi = fi.z - (float)sz;
-        int xa = x0 - 2;
-        const int xb = x1 + 2;
-        if (xa < 0) {
-          run(sst[row + m + xa], sst[row + m], fi.x + 1.0f, yi, zi);
-          xa = 0;
-        }
-        if (xb > m) {
-          run(sst[row + xa], sst[row + m], fi.x, yi, zi);
-          run(sst[row], sst[row + xb - m], fi.x - 1.0f, yi, zi);
-        } else {
-          run(sst[row + xa], sst[row + xb], fi.x, yi, zi);
-        }
+  int k = lane, ps = -1;
+  for (int z = z0; z < z1; z++)
+    for (int y = y0; y < y1; y++) {  // entry k of the brick's runs (z, y) of x0..x1-1
+      const int row = m * (y + m * z);
+      const int q0 = sst[row + x0], len = sst[row + x1] - q0;
+      if (ps < 0) {
+        if (k < len) ps = q0 + k;
+        else k -= len;
       }
     }
-    if (valid) {
-      lw.finish(lst, n, sl, maxnb);
-      const int i = d.poff + sl;
-      if (lw.n > maxnb) {
-        v.nbn[i] = -1;
-        atomicAdd(&v.st[r].overflow, 1);
-      } else {
-        v.nbn[i] = lw.n;
+  const bool valid = ps >= 0;
+  // a lane past the brick's particles gets NaN coordinates: it passes no test
+  const float4 fi = valid ? xs[ps] : make_float4(nan, nan, nan, __int_as_float(-1));
+  const int codei = __float_as_int(fi.w);
+  const int sl = codei & 0x7fff;
+  float c0, c1;
+  box_cuts(d, valid ? codei >> 15 : 0, c0, c1);
+  const uint16_t *const col = &S.col[0][lane];
+  const unsigned col0 = (unsigned)__cvta_generic_to_shared(col);
+  unsigned at = col0;  // the column's next free entry (entries 64 bytes apart)
+  int nn = 0;          // entries moved to the list
+  int u = 0;           // this lane's run
+  __syncwarp();
+  for (int f0 = 0; f0 < Q; f0 += BRICK_BATCH) {
+    float4 c[BRICK_BATCH / 32];
+#pragma unroll
+    for (int e = 0; e < BRICK_BATCH / 32; e++) {
+      const int f = f0 + 32 * e + lane;
+      c[e] = make_float4(nan, nan, nan, __int_as_float(-1));
+      if (f < Q) {
+        while (S.first[u + 1] <= f) u++;
+        c[e] = xs[S.start[u] + (f - S.first[u])];
+        const int row = u / 3;
+        c[e].x += (float)(u - 3 * row - 1);
+        c[e].y += (float)S.sy[row];
+        c[e].z += (float)S.sz[row];
       }
+    }
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < BRICK_BATCH / 32; e++) S.cand[32 * e + lane] = c[e];
+    __syncwarp();
+    // eight at a time: all their loads and distances before their appends (a
+    // store to the column keeps later loads behind it)
+#pragma unroll 1
+    for (int q = 0; q < min(BRICK_BATCH, Q - f0); q += 8) {
+      float r2[8];
+      int code[8];
+#pragma unroll
+      for (int e = 0; e < 8; e++) {
+        const float4 fj = S.cand[q + e];
+        const float ex = fi.x - fj.x, ey = fi.y - fj.y, ez = fi.z - fj.z;
+        r2[e] = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+        code[e] = __float_as_int(fj.w);
+      }
+#pragma unroll
+      for (int e = 0; e < 8; e++)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\t"
+            "setp.lt.f32 p, %1, %2;\n\t"
+            "setp.ne.and.s32 p, %3, %4, p;\n\t"
+            "@p st.shared.u16 [%0], %5;\n\t"
+            "@p add.u32 %0, %0, 64;\n\t}"
+            : "+r"(at)
+            : "f"(r2[e]), "f"(code[e] > 0x7fff ? c1 : c0), "r"(code[e]), "r"(codei), "h"((unsigned short)code[e])
+            : "memory");
+    }
+    // full chunks to the list, the rest to the front of the column
+    int from = 0;
+    for (; (int)(at - col0) - 2 * from >= 256; from += 128) {
+      if (nn + 4 <= maxnb)
+        lst[(size_t)(nn >> 2) * n + sl] =
+            make_uint2(col[from] | ((unsigned)col[from + 32] << 16), col[from + 64] | ((unsigned)col[from + 96] << 16));
+      nn += 4;
+    }
+    if (from) {
+      const uint16_t a0 = col[from], a1 = col[from + 32], a2 = col[from + 64];
+      uint16_t *const front = &S.col[0][lane];
+      front[0] = a0;
+      front[32] = a1;
+      front[64] = a2;
+      at -= 2 * from;
     }
   }
+  if (valid) {
+    // the last, partial chunk, padded with its last entry
+    const int left = (int)(at - col0) >> 6;
+    if (left && nn + left <= maxnb) {
+      const unsigned e0 = col[0], e1 = left > 1 ? col[32] : e0, e2 = left > 2 ? col[64] : e1;
+      lst[(size_t)(nn >> 2) * n + sl] = make_uint2(e0 | (e1 << 16), e2 | (e2 << 16));
+    }
+    nn += left;
+    const int i = d.poff + sl;
+    if (nn > maxnb) {
+      v.nbn[i] = -1;
+      atomicAdd(&v.st[r].overflow, 1);
+    } else {
+      v.nbn[i] = nn;
+    }
+  }
+  __syncwarp();
   // the same lists (the sub-cells within two of the particle's own, rows in
   // (z, y) order, increasing unwrapped x): the brick's neighbourhood holds
   // them, and candidates farther than two sub-cells are beyond every cut
@@ -3066,25 +3055,23 @@ __device__ __forceinline__ void box_list_particle(const View &v, const SysDesc &
     if (sst[mid] <= ps) lo = mid;
     else hi = mid - 1;
   }
-  const int sx = lo % m, sy = (lo / m) % m, sz = lo / (m * m);
-  const double iL2 = 1.0 / (d.L * d.L);
-  float lc[3];
-  for (int k = 0; k < 3; k++) lc[k] = (float)(lcut2_of(d, k) * iL2 * (1.0 + 1e-5));
+  const int cx = lo % m, cy = (lo / m) % m, cz = lo / (m * m);
   uint16_t *lst = reinterpret_cast<uint16_t *>(box_list(v, d));
   const int maxnb = v.maxnb;
   const float4 fi = xs[ps];
   const int codei = __float_as_int(fi.w);
-  const int sl = codei & 0x7fff, ti = codei >> 15;
-  const float c0 = ti == 0 ? lc[0] : lc[1], c1 = ti == 0 ? lc[1] : lc[2];
+  const int sl = codei & 0x7fff;
+  float c0, c1;
+  box_cuts(d, codei >> 15, c0, c1);
   int cnt = 0;
-  auto run = [&](int q0, int q1, float xi, float yi, float zi) {
+  auto run = [&](int q0, int q1, float wx, float wy, float wz) {
     for (int qb = q0; qb < q1; qb += 32) {
       const int q = qb + lane;
       bool ok = false;
       int code = 0;
       if (q < q1) {
         const float4 fj = xs[q];
-        const float ex = xi - fj.x, ey = yi - fj.y, ez = zi - fj.z;
+        const float ex = fi.x - (fj.x + wx), ey = fi.y - (fj.y + wy), ez = fi.z - (fj.z + wz);
         const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
         code = __float_as_int(fj.w);
         ok = r2 < ((code >> 15) ? c1 : c0) && q != ps;
@@ -3097,30 +3084,32 @@ __device__ __forceinline__ void box_list_particle(const View &v, const SysDesc &
       cnt += __popc(bal);
     }
   };
-  for (int zz = sz - 2; zz <= sz + 2; zz++) {
+  for (int zz = cz - 2; zz <= cz + 2; zz++) {
     const int wz = zz < 0 ? -1 : (zz >= m ? 1 : 0), az = zz - wz * m;
-    for (int yy = sy - 2; yy <= sy + 2; yy++) {
+    for (int yy = cy - 2; yy <= cy + 2; yy++) {
       const int wy = yy < 0 ? -1 : (yy >= m ? 1 : 0), ay = yy - wy * m;
       const int row = m * (ay + m * az);
-      // candidate image x_j + w: compare x_i - w with x_j
-      const float yi = fi.y - (float)wy, zi = fi.z - (float)wz;
-      int xa = sx - 2;
-      const int xb = sx + 3;
+      const float sy = (float)wy, sz = (float)wz;  // the candidates' image
+      int xa = cx - 2;
+      const int xb = cx + 3;
       if (xa < 0) {
-        run(sst[row + m + xa], sst[row + m], fi.x + 1.0f, yi, zi);
+        run(sst[row + m + xa], sst[row + m], -1.0f, sy, sz);
         xa = 0;
       }
       if (xb > m) {
-        run(sst[row + xa], sst[row + m], fi.x, yi, zi);
-        run(sst[row], sst[row + xb - m], fi.x - 1.0f, yi, zi);
+        run(sst[row + xa], sst[row + m], 0.0f, sy, sz);
+        run(sst[row], sst[row + xb - m], 1.0f, sy, sz);
       } else {
-        run(sst[row + xa], sst[row + xb], fi.x, yi, zi);
+        run(sst[row + xa], sst[row + xb], 0.0f, sy, sz);
       }
     }
   }
-  // the rest of the last chunk written as 0 (the force loop stops at the count)
-  if (cnt <= maxnb && lane < ((4 - (cnt & 3)) & 3))
-    lst[(((size_t)((cnt + lane) >> 2) * n + sl) << 2) + ((cnt + lane) & 3)] = 0;
+  // the rest of the last chunk repeats the last entry
+  __syncwarp();
+  if (cnt <= maxnb && (cnt & 3) && lane < 4 - (cnt & 3)) {
+    const size_t at = ((size_t)(cnt >> 2) * n + sl) << 2;
+    lst[at + (cnt & 3) + lane] = lst[at + (cnt & 3) - 1];
+  }
   if (lane == 0) {
     const int i = d.poff + sl;
     if (cnt > maxnb) {
@@ -3212,9 +3201,8 @@ __global__ void __launch_bounds__(BLOCK_SORT) k_sort_sub(View v) {
 
 
 // list bricks of a whole-box system with list sub-cells
-__device__ __forceinline__ int bricks_of(const SysDesc &d) {
-  const int nbx = (d.msub + 1) >> 1;
-  return nbx * nbx * ((d.msub + d.bz - 1) / d.bz);
+__device__ __forceinline__ int bricks_of(const SysDesc &d, int bx, int bz) {
+  return ((d.msub + bx - 1) / bx) * ((d.msub + 1) >> 1) * ((d.msub + bz - 1) / bz);
 }
 
 // one block: the whole-box systems with list sub-cells that rebuild this step,
@@ -3234,7 +3222,7 @@ __global__ void __launch_bounds__(BLOCK_COMPACT) k_rebuild_compact(View v) {
       const SysDesc &d = v.desc[r];
       if (v.st[r].rebuild && d.box && d.msub >= 5) {
         f = 1;
-        nb = v.box_warp ? d.n : bricks_of(d);
+        nb = v.box_warp ? d.n : bricks_of(d, 2, d.bz);
       }
     }
     // block-wide exclusive scans of the flags and brick counts
@@ -3285,6 +3273,7 @@ __global__ void __launch_bounds__(BLOCK_COMPACT) k_rebuild_compact(View v) {
 __global__ void __launch_bounds__(BLOCK_X) k_build_list_box(View v) {
   extern __shared__ float4 xstg[];
   __shared__ int cst[MAX_BOX_CELLS + 1], pre4[MAX_BOX_CELLS + 1];
+  __shared__ BrickScratch buf[BLOCK_X / 32];
   const int2 tile = v.tiles_x[blockIdx.x / LIST_SPLIT];
   const int part = blockIdx.x % LIST_SPLIT;
   const int r = tile.x, b = tile.y;
@@ -3329,7 +3318,8 @@ __global__ void __launch_bounds__(BLOCK_X) k_build_list_box(View v) {
     if (v.box_warp)
       box_list_particle(v, ds, rs, v.xsub + ds.poff, v.ssub + ds.soff, it - v.rbs[3 + 2 * lo], lane);
     else
-      box_list_brick(v, ds, rs, v.xsub + ds.poff, v.ssub + ds.soff, it - v.rbs[3 + 2 * lo], lane);
+      box_list_brick(v, ds, rs, v.xsub + ds.poff, v.ssub + ds.soff, it - v.rbs[3 + 2 * lo], 2, ds.bz, lane,
+                     buf[warp]);
   }
 }
 
@@ -3367,7 +3357,6 @@ __device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, co
   const int *qx = reinterpret_cast<const int *>(xsm), *qy = qx + n, *qz = qy + n;
   const double *sx = reinterpret_cast<const double *>(xsm), *sy = sx + n, *sz = sy + n;
   const double L = d.L;
-  const float scale = (float)(L * (1.0 / 4294967296.0));
   {
     PairAcc a = {0.0, 0.0, 0.0, 0.0, 0.0};
     if (valid && nn >= 0) {
@@ -3376,41 +3365,37 @@ __device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, co
       if (PREC == 1) {
         // separations in fixed-point units (L / 2^32), folded into the constants
         const unsigned xi = qx[sl], yi = qy[sl], zi = qz[sl];
-        const PairParamsF P(ti, scale);
-        PairAccF fa = {0.f, 0.f, 0.f, 0.f, 0.f}, fb = {0.f, 0.f, 0.f, 0.f, 0.f};
+        const PairParamsF P(ti, L * (1.0 / 4294967296.0));
         for (int c = lane; c < nch; c += TPP) {
           const uint2 wn = c + TPP < nch ? lp[(size_t)(c + TPP) * stride] : make_uint2(0u, 0u);
-          const int k0 = 4 * c;
+          const int left = nn - 4 * c;
+          PairAccF f = {0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll
           for (int e = 0; e < 4; e++) {
-            const int code = ((e < 2 ? w.x : w.y) >> (16 * (e & 1))) & 0xffff;
-            if (e == 0 || k0 + e < nn) {
-              const int j = code & 0x7fff;
-              const float dx = (float)(int)(xi - (unsigned)qx[j]);
-              const float dy = (float)(int)(yi - (unsigned)qy[j]);
-              const float dz = (float)(int)(zi - (unsigned)qz[j]);
-              pair_f32(e & 1 ? fb : fa, dx, dy, dz, P, code >> 15);
-            }
+            const unsigned code = ((e < 2 ? w.x : w.y) >> (16 * (e & 1))) & 0xffffu;
+            const unsigned j = code & 0x7fffu;
+            const float dx = (float)(int)(xi - (unsigned)qx[j]);
+            const float dy = (float)(int)(yi - (unsigned)qy[j]);
+            const float dz = (float)(int)(zi - (unsigned)qz[j]);
+            pair_f32(f, dx, dy, dz, P, code >> 15, e < left);
           }
-          flush_chunk(fa, fb, a);
+          flush_chunk(f, a);
           w = wn;
         }
-        a.vir *= (double)scale;
+        pair_scale(a, L * (1.0 / 4294967296.0));
       } else {
         const double xi = sx[sl], yi = sy[sl], zi = sz[sl];
-        const PairParamsD P(ti);
+        const PairParamsD P(ti, L);
         PairAcc bb = {0.0, 0.0, 0.0, 0.0, 0.0};
         for (int c = lane; c < nch; c += TPP) {
           const uint2 wn = c + TPP < nch ? lp[(size_t)(c + TPP) * stride] : make_uint2(0u, 0u);
-          const int k0 = 4 * c;
+          const int left = nn - 4 * c;
 #pragma unroll
           for (int e = 0; e < 4; e++) {
-            const int code = ((e < 2 ? w.x : w.y) >> (16 * (e & 1))) & 0xffff;
-            if (e == 0 || k0 + e < nn) {
-              const int q = code & 0x7fff;
-              pair_f64(e & 1 ? bb : a, min_image(xi - sx[q]) * L, min_image(yi - sy[q]) * L,
-                       min_image(zi - sz[q]) * L, P, code >> 15);
-            }
+            const unsigned code = ((e < 2 ? w.x : w.y) >> (16 * (e & 1))) & 0xffffu;
+            const unsigned q = code & 0x7fffu;
+            pair_f64(e & 1 ? bb : a, min_image(xi - sx[q]), min_image(yi - sy[q]), min_image(zi - sz[q]), P,
+                     code >> 15, e < left);
           }
           w = wn;
         }
@@ -3419,6 +3404,7 @@ __device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, co
         a.fz += bb.fz;
         a.pe += bb.pe;
         a.vir += bb.vir;
+        pair_scale(a, L);
       }
     } else if (valid) {
       // list overflow: all particles of the 27 neighbour images (each pair once)

@@ -27,8 +27,8 @@
 //
 // What bounds it: the latency of a step's dependent phases for a lone system
 // (16 of 148 SMs busy), the issue rate of the pair terms for a batch.  Measured
-// on B200 against the kernel-by-kernel graphs: N = 1000 FP64 39.0 -> 21.8 us a
-// step, N = 4000 FP64 60 -> 43, 256 FP32 replicas 400 -> 278.
+// on B200 against the kernel-by-kernel graphs: N = 1000 FP64 39.0 -> 15.1 us a
+// step, N = 4000 FP64 60 -> 38, 256 FP32 replicas 400 -> 245.
 //
 // Sums, lists and particle order are those of the kernel-by-kernel step, so a
 // system's results are the same bits whichever path, cluster size or residency
@@ -47,18 +47,19 @@ constexpr size_t RUN_SMEM_MAX = 219 * 1024;           // dynamic; the static arr
 
 __host__ __device__ __forceinline__ size_t run_align(size_t x) { return (x + 15) & ~(size_t)15; }
 
-// shared-memory plan of one system on a cluster of C blocks (byte offsets)
+// shared-memory plan of one system on a cluster of C blocks of nw warps (byte offsets)
 struct RunPlan {
   int nseg, nloc;       // 32-slot segments; slots per block
   size_t seg8, nn, state;  // this block's sums per 8 slots, list lengths and slots' state (none when not resident)
   size_t pool;          // staging and list cache, or the rebuild's scratch
   size_t stage_bytes, scratch_bytes, perm_bytes;
+  size_t lists_at;      // in the scratch: the sorts' arrays, then the list buffers
   // the least dynamic shared memory
   __host__ __device__ size_t least() const {
     return pool + (stage_bytes > scratch_bytes ? stage_bytes : scratch_bytes) + perm_bytes;
   }
 };
-__host__ __device__ __forceinline__ RunPlan run_plan(int n, int ncell, int msub, int prec, int C, bool resident) {
+__host__ __device__ __forceinline__ RunPlan run_plan(int n, int ncell, int msub, int prec, int C, bool resident, int nw) {
   RunPlan p;
   p.nseg = (n + 31) / 32;
   p.nloc = 32 * ((p.nseg + C - 1) / C);
@@ -68,10 +69,13 @@ __host__ __device__ __forceinline__ RunPlan run_plan(int n, int ncell, int msub,
   p.pool = p.state + (resident ? run_align((size_t)RUN_STATE_BYTES * p.nloc) : 0);
   p.stage_bytes = run_align((size_t)n * (prec ? 12 : 24));
   const size_t m3 = (size_t)msub * msub * msub, hist = 64 * (size_t)ncell, xs = 16 * (size_t)n;
-  // cell or sub-cell key and order per slot, sub-cell counts and starts, then
   // the sorted candidates (or the cell sort's per-warp counts and cell starts)
-  p.scratch_bytes = 2 * run_align(2 * (size_t)n) + 2 * run_align(4 * (m3 + 1)) +
-                    run_align(xs > hist + 4 * (size_t)ncell ? xs : hist + 4 * (size_t)ncell);
+  // and the sub-cell starts; then the sorts' keys, orders and counts or, once
+  // those are done, the list buffers of as many warps as there is room for (at
+  // least half of them)
+  const size_t sort = 2 * run_align(2 * (size_t)n) + run_align(4 * m3), lists = sizeof(BrickScratch) * (nw / 2);
+  p.lists_at = run_align(xs > hist + 4 * (size_t)ncell ? xs : hist + 4 * (size_t)ncell) + run_align(4 * (m3 + 1));
+  p.scratch_bytes = p.lists_at + (sort > lists ? sort : lists);
   p.perm_bytes = run_align(2 * (size_t)n);
   return p;
 }
@@ -234,7 +238,7 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
   __shared__ SysDesc sd;
   __shared__ double s_wmax[32], s_cmax[RUN_MAX_CLUSTER];
   __shared__ double s_obs[OBS_EMAX][OBS_NV];
-  __shared__ int s_nnmax;
+  __shared__ int s_nnmax, s_brick;
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
   const int r = order[blockIdx.x / C];
@@ -248,7 +252,7 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
   copy_struct(&sd, &v.desc[r]);
   __syncthreads();
   const int n = sd.n, poff = sd.poff;
-  const RunPlan P = run_plan(n, sd.ncell, sd.msub, PREC, C, RES);
+  const RunPlan P = run_plan(n, sd.ncell, sd.msub, PREC, C, RES, NW);
   const int lo = rank * P.nloc, hi = max(lo, min(n, lo + P.nloc)), own = hi - lo;
   const int lo_seg = rank * (P.nloc / 32), nseg_own = max(0, min(P.nseg - lo_seg, P.nloc / 32));
   double4 *seg = reinterpret_cast<double4 *>(rsm), *seg8 = reinterpret_cast<double4 *>(rsm + P.seg8);
@@ -356,17 +360,19 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
       ss.force_rebuild = 0;
     }
     if (rebuild) {
-      uint16_t *key = reinterpret_cast<uint16_t *>(stg);
-      uint16_t *ord = reinterpret_cast<uint16_t *>(stg + run_align(2 * (size_t)n));
       const int m3 = sd.msub * sd.msub * sd.msub;
-      int *fill = reinterpret_cast<int *>(stg + 2 * run_align(2 * (size_t)n));
-      int *sst = reinterpret_cast<int *>(stg + 2 * run_align(2 * (size_t)n) + run_align(4 * (size_t)(m3 + 1)));
-      float4 *xs = reinterpret_cast<float4 *>(stg + 2 * run_align(2 * (size_t)n) + 2 * run_align(4 * (size_t)(m3 + 1)));
+      float4 *xs = reinterpret_cast<float4 *>(stg);
+      int *sst = reinterpret_cast<int *>(stg + P.lists_at - run_align(4 * (size_t)(m3 + 1)));
+      uint16_t *key = reinterpret_cast<uint16_t *>(stg + P.lists_at);
+      uint16_t *ord = reinterpret_cast<uint16_t *>(stg + P.lists_at + run_align(2 * (size_t)n));
+      int *fill = reinterpret_cast<int *>(stg + P.lists_at + 2 * run_align(2 * (size_t)n));
+      BrickScratch *buf = reinterpret_cast<BrickScratch *>(stg + P.lists_at);
       if (RES) {  // the state in global memory, for the blocks that take over its slots
         for (int k = lo + tid; k < hi; k += NT) run_copy_slot(g, poff + k, w, wb + k);
       }
       if (tid == 0) {
         ss.rebuilds += 1;
+        s_brick = 0;
         if (rank == 0) v.st[r].overflow = 0;
       }
       bar();
@@ -383,13 +389,17 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
       }
       sort_sub_cells(n, sd.msub, [&](int s) { return v.pos[poff + perm[s]]; }, fill, sst, key, ord, xs);
       __syncthreads();
-      // lists: one warp per particle (short chains) while a warp gets few
-      // particles, else one lane per particle over bricks (fewer instructions)
-      if (n <= 8 * C * NW) {
-        for (int q = rank * NW + warp; q < n; q += C * NW) box_list_particle(v, sd, r, xs, sst, q, lane);
-      } else {
-        const int nb = bricks_of(sd);
-        for (int q = rank * NW + warp; q < nb; q += C * NW) box_list_brick(v, sd, r, xs, sst, q, lane);
+      // lists, one brick of sub-cells a warp: the smaller ones where the cluster
+      // has warps to spare, else as many lanes of a sweep in use as fit
+      const int bx = C > 1 ? 2 : sd.bx_wide, nb = bricks_of(sd, bx, sd.bz);
+      const int lw = min(NW, (int)((smem_bytes - P.perm_bytes - P.pool - P.lists_at) / sizeof(BrickScratch)));
+      if (C > 1) {
+        if (warp < lw)
+          for (int q = warp * C + rank; q < nb; q += C * lw)
+            box_list_brick(v, sd, r, xs, sst, q, bx, sd.bz, lane, buf[warp]);
+      } else if (warp < lw) {  // several bricks a warp: handed out as warps come free
+        for (int q = warp_next(s_brick); q < nb; q = warp_next(s_brick))
+          box_list_brick(v, sd, r, xs, sst, q, bx, sd.bz, lane, buf[warp]);
       }
       __syncthreads();
       for (int s = tid; s < n; s += NT) run_stage<PREC>(stg, n, s, v.pos[poff + perm[s]]);
