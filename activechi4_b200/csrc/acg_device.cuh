@@ -261,6 +261,85 @@ __device__ __forceinline__ int wrap_cell(int c, int nc) {
   return c >= nc ? (c >= 2 * nc ? c - 2 * nc : c - nc) : c;
 }
 
+// sums over one particle's pairs
+struct PairAcc {
+  double fx, fy, fz, pe, vir;
+};
+
+// 1/x for x in the pair range (0.3 < x < 7): the hardware estimate
+// (rcp.approx.ftz.f64, relative error e below 2^-20) refined by one step of
+// Halley's third-order iteration, y (1 + e + e^2) with e = 1 - x y: the error
+// becomes e^3, below the rounding, in three operations
+__device__ __forceinline__ double rcp_nr(double x) {
+  double y;
+  asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
+}
+
+// 1/sigma^2 and 4 eps of a pair by its type sum (MDcode/cell_list+forces.c:19-20)
+__device__ __forceinline__ double ka_is2(int tp) { return tp == 0 ? 1.0 : (tp == 1 ? 1.5625 : 1.0 / (0.88 * 0.88)); }
+__device__ __forceinline__ double ka_e4(int tp) { return tp == 0 ? 4.0 : (tp == 1 ? 6.0 : 2.0); }
+
+// The pair terms below take separations counted in units u of length (u^2 is
+// folded into 1/sigma^2) and add up pe, h d and h d^2 with
+// h = 4 eps u^2/sigma^2 (s6 (6 s6 - 3) s2 - C2), half of the radial force factor
+// times u^2: in absolute units the force is 2/u and the virial 2 times the sums
+// (pair_scale).  Everything is evaluated for every list entry and masked by a
+// zero 4 eps beyond the cut or the list's end (no divergent branch: the entries
+// of a chunk interleave, and each sum gains exactly nothing; the entries that
+// pad a list repeat its last one or lie far away, so every term is finite).
+__device__ __forceinline__ void pair_scale(PairAcc &a, double u) {
+  const double c = 2.0 / u;
+  a.fx *= c;
+  a.fy *= c;
+  a.fz *= c;
+  a.vir *= 2.0;
+}
+
+// FP64 pair constants; 4 eps by its high word (4, 6 and 2 have an empty low one)
+struct PairParamsD {
+  double is2[2];
+  int e4hi[2];
+  __device__ __forceinline__ PairParamsD(int ti, double u) {
+#pragma unroll
+    for (int tj = 0; tj < 2; tj++) {
+      is2[tj] = ka_is2(ti + tj) * (u * u);
+      e4hi[tj] = __double2hiint(ka_e4(ti + tj));
+    }
+  }
+};
+
+// FP64 pair term (MDcode/cell_list+forces.c:174-203), in fused multiply-adds
+__device__ __forceinline__ void pair_f64(PairAcc &a, double dx, double dy, double dz, const PairParamsD &P,
+                                         bool tj, bool valid) {
+  const double is2 = tj ? P.is2[1] : P.is2[0];
+  const double dr2 = fma(dx, dx, fma(dy, dy, dz * dz));
+  const double rs2 = dr2 * is2;
+  const bool in = rs2 < KA_RC2 && valid;
+  const double e4 = __hiloint2double(in ? (tj ? P.e4hi[1] : P.e4hi[0]) : 0, 0);
+  const double s2 = rcp_nr(rs2);
+  const double s6 = s2 * s2 * s2;
+  a.pe = fma(e4, fma(s6, s6, -s6) + fma(KA_C2, rs2, KA_C0), a.pe);
+  const double g = (e4 * is2) * fma(s6 * fma(6.0, s6, -3.0), s2, -KA_C2);
+  a.fx = fma(g, dx, a.fx);
+  a.fy = fma(g, dy, a.fy);
+  a.fz = fma(g, dz, a.fz);
+  a.vir = fma(g, dr2, a.vir);
+}
+
+// the union cell holding staged index q: the last u with pre[u] <= q (pre is a
+// non-decreasing prefix over n cells in shared memory)
+__device__ __forceinline__ int union_of(const int *pre, int n, int q) {
+  int lo = 0, hi = n - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (pre[mid] <= q) lo = mid;
+    else hi = mid - 1;
+  }
+  return lo;
+}
+
 // U4Propagator (MDcode/time_evolve.c:578-609): one chain sweep jStart..jEnd,
 // `ksum` = sum p^2 for the j == 0 link.
 __device__ inline void nhc_u4(double *p_eta, const double *q, double T, double dof, double t,

@@ -18,6 +18,7 @@
 // device) race on the array and must be serialised by the caller.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 #include <string>
 
@@ -30,10 +31,14 @@ int set_last_error(int code, const std::string &msg);  // acg_engine.cu: the tex
 
 namespace {
 
-constexpr int NA_BLOCK = 128;
-constexpr int NA_TPP = 4;
-constexpr int NA_PB = NA_BLOCK / NA_TPP;  // particles per force block
-constexpr int NA_MAX_BLOCKS = (ACG_NOALLOC_MAX_N + NA_PB - 1) / NA_PB;
+constexpr int NA_BLOCK = 256;
+constexpr int NA_WARPS = NA_BLOCK / 32;
+constexpr int NA_MAX_BLOCKS = 8192;  // force blocks (each takes every NA_MAX_BLOCKS-th cell)
+// candidates of a cell's neighbourhood staged in shared memory: at density 1.2
+// a neighbourhood of 27 cells holds 750 to 1000 (up to 1250 where cells are
+// widest); with 40 bytes each four blocks of eight warps share an SM
+constexpr int NA_CAP = 1280;
+constexpr size_t NA_SMEM = (size_t)NA_CAP * (sizeof(float4) + 3 * sizeof(double));
 
 // scratch layout (bytes): cell_of[N] order[N] ccount[C] cstart[C] cfill[C]
 // partials[B][4] counter
@@ -119,103 +124,183 @@ __global__ void k_na_scatter(NaArgs a) {
   na_i(a, OFF_ORDER)[slot] = i;
 }
 
-// KA pair term, as MDcode/cell_list+forces.c:174-203 (each pair seen from
-// both sides, so energy and virial are halved at the end)
-__device__ __forceinline__ void na_pair(double xi, double yi, double zi, int ti, const NaArgs &a, int j,
-                                        double &fx, double &fy, double &fz, double &pe, double &vir) {
-  const double L = a.L;
-  const double dx = acg::min_image(xi - a.x[3 * j]), dy = acg::min_image(yi - a.x[3 * j + 1]),
-               dz = acg::min_image(zi - a.x[3 * j + 2]);
-  const double dr2 = (dx * dx + dy * dy + dz * dz) * L * L;
-  const int tp = ti + a.type[j];
-  const double is2 = tp == 0 ? 1.0 : (tp == 1 ? 1.5625 : 1.0 / (0.88 * 0.88));
-  const double rs2 = dr2 * is2;
-  if (rs2 < acg::KA_RC2) {
-    const double e4 = tp == 0 ? 4.0 : (tp == 1 ? 6.0 : 2.0);
-    const double s2 = 1.0 / rs2, s6 = s2 * s2 * s2;
-    pe += e4 * ((s6 * (s6 - 1.0)) + acg::KA_C0 + acg::KA_C2 * rs2);
-    const double g = (2.0 * e4 * is2) * (6.0 * s6 * (s6 - 0.5) * s2 - acg::KA_C2);
-    fx += g * L * dx;
-    fy += g * L * dy;
-    fz += g * L * dz;
-    vir += g * dr2;
-  }
-}
-
-__global__ void __launch_bounds__(NA_BLOCK) k_na_force(NaArgs a) {
-  __shared__ double sh[4][NA_BLOCK / 32];
+// Forces by cells: one block stages a cell's 27 neighbour cells (8 at two cells
+// per side) once -- FP32 reduced coordinates with index and type for the
+// distance test, FP64 ones for the pair terms -- and its warps take the cell's
+// particles one at a time: the lanes test 32 candidates a step in FP32 against
+// the pair's own cut widened by 1e-4 (the coordinates' rounding is below 2e-5 of
+// it at the largest box), the accepted ones queue up, and every 32 of them are
+// evaluated by a full warp in FP64 (masked by the exact cut).  About one
+// candidate in twelve is within the cut, so the FP64 terms, which bounded a
+// version that evaluated each candidate under a branch, run on full warps.
+// What bounds it now: issue (about 50 instructions per 32 candidates tested).
+// N = 20000: 260 -> 100 us a call with the cell build.
+// A neighbourhood above NA_CAP candidates is evaluated straight from memory.
+__global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
+  extern __shared__ __align__(16) unsigned char na_sm[];
+  float4 *cf = reinterpret_cast<float4 *>(na_sm);
+  double *cx = reinterpret_cast<double *>(na_sm + NA_CAP * sizeof(float4)), *cy = cx + NA_CAP, *cz = cy + NA_CAP;
+  __shared__ int s_pre[28], s_start[27];
+  __shared__ uint16_t queue[NA_WARPS][96];
+  __shared__ signed char s_img[3][27];  // image of each neighbour cell (3 and more cells per side)
+  __shared__ double sh[3][NA_WARPS];
   __shared__ int s_last;
-  const int grp = threadIdx.x / NA_TPP, lane = threadIdx.x % NA_TPP;
-  const int i = blockIdx.x * NA_PB + grp;
-  const bool valid = i < a.n;
-  double fx = 0, fy = 0, fz = 0, pe = 0, vir = 0;
-  if (valid) {
-    const double xi = a.x[3 * i], yi = a.x[3 * i + 1], zi = a.x[3 * i + 2];
-    const int ti = a.type[i];
-    const int nc = a.nc, c = na_i(a, OFF_CELL)[i];
-    const int cx = c % nc, cy = (c / nc) % nc, cz = c / (nc * nc);
-    const int lo = acg::stencil_lo(nc), hi = acg::stencil_hi(nc);
-    for (int oz = lo; oz <= hi; oz++)
-      for (int oy = lo; oy <= hi; oy++)
-        for (int ox = lo; ox <= hi; ox++) {
-          const int c2 = acg::wrap_cell(cx + ox, nc) + acg::wrap_cell(cy + oy, nc) * nc +
-                         acg::wrap_cell(cz + oz, nc) * nc * nc;
-          const int s0 = na_i(a, OFF_START)[c2], m = na_i(a, OFF_COUNT)[c2];
-          for (int q = lane; q < m; q += NA_TPP) {
-            const int j = na_i(a, OFF_ORDER)[s0 + q];
-            if (j != i) na_pair(xi, yi, zi, ti, a, j, fx, fy, fz, pe, vir);
-          }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int nc = a.nc, ncell = nc * nc * nc;
+  const int lo = acg::stencil_lo(nc), wd = acg::stencil_hi(nc) - lo + 1, ns = wd * wd * wd;
+  const int own = nc >= 3 ? 13 : 0;  // the cell itself among its neighbours
+  const double L = a.L;
+  const int *order = na_i(a, OFF_ORDER);
+  float cut[3];  // the test's cuts by type sum, reduced units
+  for (int k = 0; k < 3; k++) cut[k] = (float)(acg::KA_RC2 * (1.0 + 1e-4) / (acg::ka_is2(k) * L * L));
+  double sum[3] = {0.0, 0.0, 0.0};  // pe, virial, active virial of this warp's particles (lane 0)
+  for (int c = blockIdx.x; c < ncell; c += gridDim.x) {
+    if (warp == 0) {
+      int m = 0;
+      if (lane < ns) {
+        const int cc[3] = {c % nc + lane % wd + lo, (c / nc) % nc + (lane / wd) % wd + lo,
+                           c / (nc * nc) + lane / (wd * wd) + lo};
+        int c2 = 0, mul = 1;
+        for (int k = 0; k < 3; k++, mul *= nc) {
+          c2 += acg::wrap_cell(cc[k], nc) * mul;
+          s_img[k][lane] = (signed char)(nc < 3 ? 0 : (cc[k] < 0 ? -1 : (cc[k] >= nc ? 1 : 0)));
         }
-  }
-#pragma unroll
-  for (int o = NA_TPP / 2; o > 0; o >>= 1) {
-    fx += __shfl_xor_sync(0xffffffffu, fx, o);
-    fy += __shfl_xor_sync(0xffffffffu, fy, o);
-    fz += __shfl_xor_sync(0xffffffffu, fz, o);
-    pe += __shfl_xor_sync(0xffffffffu, pe, o);
-    vir += __shfl_xor_sync(0xffffffffu, vir, o);
-  }
-  double va = 0.0;
-  if (valid && lane == 0) {
-    const int t = a.act[i];
-    if (t >= 0 && t < a.nact) {  // active force (MDcode/cell_list+forces.c:207-218)
-      const double kx = (double)a.k[t], ky = (double)a.k[a.nact + t], kz = (double)a.k[2 * a.nact + t];
-      const double *u = a.xu ? a.xu : a.x;
-      fx += a.f0 * kx;
-      fy += a.f0 * ky;
-      fz += a.f0 * kz;
-      va = a.f0 * (kx * u[3 * i] + ky * u[3 * i + 1] + kz * u[3 * i + 2]);
+        s_start[lane] = na_i(a, OFF_START)[c2];
+        m = na_i(a, OFF_COUNT)[c2];
+      }
+      int x = m;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane < ns) s_pre[lane + 1] = x;
+      if (lane == 0) s_pre[0] = 0;
     }
-    a.F[3 * i] = fx;
-    a.F[3 * i + 1] = fy;
-    a.F[3 * i + 2] = fz;
+    __syncthreads();
+    const int Q = s_pre[ns], mc = s_pre[own + 1] - s_pre[own];
+    const bool staged = Q <= NA_CAP;
+    if (staged && mc > 0)
+      for (int q = threadIdx.x; q < Q; q += NA_BLOCK) {
+        const int u = acg::union_of(s_pre, ns, q);
+        const int j = order[s_start[u] + (q - s_pre[u])];
+        const double x = a.x[3 * j], y = a.x[3 * j + 1], z = a.x[3 * j + 2];
+        cf[q] = make_float4((float)(x + s_img[0][u]), (float)(y + s_img[1][u]), (float)(z + s_img[2][u]),
+                            __int_as_float(j | (a.type[j] << 30)));
+        cx[q] = x;
+        cy[q] = y;
+        cz[q] = z;
+      }
+    __syncthreads();
+    for (int w = warp; w < mc; w += NA_WARPS) {
+      const int i = order[s_start[own] + w];
+      const int ti = a.type[i];
+      const acg::PairParamsD P(ti, L);
+      acg::PairAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+      if (staged) {
+        const int qi = s_pre[own] + w;
+        const float4 fi = cf[qi];
+        const double xi = cx[qi], yi = cy[qi], zi = cz[qi];
+        const float c0 = ti == 0 ? cut[0] : cut[1], c1 = ti == 0 ? cut[1] : cut[2];
+        uint16_t *qu = queue[warp];
+        int cnt = 0;
+        auto pairs = [&](int k) {  // the last k <= 32 of the queue
+          __syncwarp();
+          cnt -= k;
+          const int q = qu[cnt + (lane < k ? lane : 0)];
+          acg::pair_f64(acc, acg::min_image(xi - cx[q]), acg::min_image(yi - cy[q]), acg::min_image(zi - cz[q]), P,
+                        (__float_as_int(cf[q].w) >> 30) & 1, lane < k);
+          __syncwarp();
+        };
+        auto test = [&](int q) {
+          if (q >= Q) return false;
+          const float4 fj = cf[q];
+          float dx = fi.x - fj.x, dy = fi.y - fj.y, dz = fi.z - fj.z;
+          if (nc < 3) {  // every cell neighbours every other under two images
+            dx -= rintf(dx);
+            dy -= rintf(dy);
+            dz -= rintf(dz);
+          }
+          return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < (((__float_as_int(fj.w) >> 30) & 1) ? c1 : c0) && q != qi;
+        };
+        const unsigned below = (1u << lane) - 1u;
+        for (int q0 = lane; q0 - lane < Q; q0 += 64) {
+          const bool ok0 = test(q0), ok1 = test(q0 + 32);
+          const unsigned b0 = __ballot_sync(0xffffffffu, ok0), b1 = __ballot_sync(0xffffffffu, ok1);
+          if (ok0) qu[cnt + __popc(b0 & below)] = (uint16_t)q0;
+          cnt += __popc(b0);
+          if (ok1) qu[cnt + __popc(b1 & below)] = (uint16_t)(q0 + 32);
+          cnt += __popc(b1);
+          while (cnt >= 32) pairs(32);
+        }
+        if (cnt > 0) pairs(cnt);
+      } else {
+        const double xi = a.x[3 * i], yi = a.x[3 * i + 1], zi = a.x[3 * i + 2];
+        for (int u = 0; u < ns; u++)
+          for (int q = lane; q < s_pre[u + 1] - s_pre[u]; q += 32) {
+            const int j = order[s_start[u] + q];
+            if (j != i)
+              acg::pair_f64(acc, acg::min_image(xi - a.x[3 * j]), acg::min_image(yi - a.x[3 * j + 1]),
+                            acg::min_image(zi - a.x[3 * j + 2]), P, a.type[j] != 0, true);
+          }
+      }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        acc.fx += __shfl_xor_sync(0xffffffffu, acc.fx, o);
+        acc.fy += __shfl_xor_sync(0xffffffffu, acc.fy, o);
+        acc.fz += __shfl_xor_sync(0xffffffffu, acc.fz, o);
+        acc.pe += __shfl_xor_sync(0xffffffffu, acc.pe, o);
+        acc.vir += __shfl_xor_sync(0xffffffffu, acc.vir, o);
+      }
+      if (lane == 0) {
+        acg::pair_scale(acc, L);
+        const int t = a.act[i];
+        if (t >= 0 && t < a.nact) {  // active force (MDcode/cell_list+forces.c:207-218)
+          const double kx = (double)a.k[t], ky = (double)a.k[a.nact + t], kz = (double)a.k[2 * a.nact + t];
+          const double *u = a.xu ? a.xu : a.x;
+          acc.fx += a.f0 * kx;
+          acc.fy += a.f0 * ky;
+          acc.fz += a.f0 * kz;
+          sum[2] += a.f0 * (kx * u[3 * i] + ky * u[3 * i + 1] + kz * u[3 * i + 2]);
+        }
+        a.F[3 * i] = acc.fx;
+        a.F[3 * i + 1] = acc.fy;
+        a.F[3 * i + 2] = acc.fz;
+        sum[0] += acc.pe;
+        sum[1] += acc.vir;
+      }
+    }
+    __syncthreads();
   }
-  if (lane != 0 || !valid) pe = vir = 0.0;
-  double v3[3] = {pe, vir, va};
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  for (int q = 0; q < 3; q++) {
-    double s = v3[q];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if (l == 0) sh[q][w] = s;
-  }
+  if (lane == 0)
+    for (int q = 0; q < 3; q++) sh[q][warp] = sum[q];
   __syncthreads();
   double *part = (double *)(a.scr + OFF_PART);
   if (threadIdx.x == 0) {
-    double t[3] = {0, 0, 0};
-    for (int q = 0; q < 3; q++)
-      for (int ww = 0; ww < NA_BLOCK / 32; ww++) t[q] += sh[q][ww];
-    part[4 * blockIdx.x] = t[0];
-    part[4 * blockIdx.x + 1] = t[1];
-    part[4 * blockIdx.x + 2] = t[2];
+    for (int q = 0; q < 3; q++) {
+      double t = 0.0;
+      for (int ww = 0; ww < NA_WARPS; ww++) t += sh[q][ww];
+      part[4 * blockIdx.x + q] = t;
+    }
     __threadfence();
     s_last = atomicAdd((unsigned int *)(a.scr + OFF_CTR), 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (!s_last || threadIdx.x != 0) return;
+  if (!s_last) return;
   __threadfence();
-  double t[3] = {0, 0, 0};
-  for (unsigned int b = 0; b < gridDim.x; b++)
+  // the last block adds up all blocks' sums
+  double t[3] = {0.0, 0.0, 0.0};
+  for (unsigned int b = threadIdx.x; b < gridDim.x; b += NA_BLOCK)
     for (int q = 0; q < 3; q++) t[q] += __ldcg(&part[4 * b + q]);
+  for (int q = 0; q < 3; q++) {
+    for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_down_sync(0xffffffffu, t[q], o);
+    if (lane == 0) sh[q][warp] = t[q];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int q = 0; q < 3; q++) {
+    t[q] = 0.0;
+    for (int ww = 0; ww < NA_WARPS; ww++) t[q] += sh[q][ww];
+  }
   a.out[0] = 0.5 * t[0];
   a.out[1] = (0.5 * t[1]) / 3.0;
   a.out[2] = t[2];
@@ -256,6 +341,11 @@ extern "C" int acg_forces_noalloc(const double *x, const double *xu, const int *
       if (ce != cudaSuccess || !p)
         return na_fail(ACG_ERR_CUDA,
                        std::string("acg_forces_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(ce));
+      // the force kernel's staging is above the default limit
+      ce = cudaFuncSetAttribute(k_na_force, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)NA_SMEM);
+      if (ce != cudaSuccess)
+        return na_fail(ACG_ERR_CUDA,
+                       std::string("acg_forces_noalloc: cudaFuncSetAttribute: ") + cudaGetErrorString(ce));
       na_ptr[dev] = p;
     }
     scr = na_ptr[dev];
@@ -281,7 +371,7 @@ extern "C" int acg_forces_noalloc(const double *x, const double *xu, const int *
   k_na_count<<<(n + 255) / 256, 256, 0, s>>>(a);
   k_na_scan<<<1, 1024, 0, s>>>(a);
   k_na_scatter<<<(n + 255) / 256, 256, 0, s>>>(a);
-  k_na_force<<<(n + NA_PB - 1) / NA_PB, NA_BLOCK, 0, s>>>(a);
+  k_na_force<<<std::min(ncell, NA_MAX_BLOCKS), NA_BLOCK, NA_SMEM, s>>>(a);
   ce = cudaGetLastError();
   if (ce != cudaSuccess)
     return na_fail(ACG_ERR_CUDA, std::string("acg_forces_noalloc: launch: ") + cudaGetErrorString(ce));
