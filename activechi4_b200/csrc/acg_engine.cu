@@ -256,6 +256,7 @@ struct acg_engine {
   int2 *d_tiles_b = nullptr;
   int2 *d_tiles_x = nullptr;
   std::vector<int> dirty;  // systems whose forces/lists must be recomputed
+  std::vector<char> loaded;  // systems that hold a state (the others wait for theirs before they are primed)
   // the host's copy of each system's step counter and ramp steps left (the
   // device's st.step / st.ramp_left), to schedule drift removals between
   // graph launches
@@ -701,7 +702,7 @@ int launch_step_eager(acg_engine *e) {
 int prime(acg_engine *e) {
   if (!e->any_dirty) return ACG_OK;
   for (int r = 0; r < e->lay.nsys; r++) {
-    if (!e->dirty[r]) continue;
+    if (!e->dirty[r] || !e->loaded[r]) continue;
     int one = 1;
     CK(cudaMemcpyAsync(&e->v.st[r].prime, &one, sizeof(int), cudaMemcpyHostToDevice, e->stream));
     e->dirty[r] = 0;
@@ -1267,12 +1268,13 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
   rc = build_tiles_b(e);
   if (rc) return cleanup_fail(rc);
   e->dirty.assign(nsys, 1);
+  e->loaded.assign(nsys, 0);
   e->hstep.assign(nsys, 0);
   e->hramp.assign(nsys, 0);
   e->obs_bufs.assign(nsys, {});
   e->obs_offsets.assign(nsys, {});
   e->obs_events.assign(nsys, {});
-  e->any_dirty = true;
+  e->any_dirty = false;
   if (cudaStreamSynchronize(e->stream) != cudaSuccess)
     return cleanup_fail(fail(ACG_ERR_CUDA, "set-up synchronisation failed"));
   *out = e;
@@ -1369,6 +1371,7 @@ int acg_set_state(acg_engine *e, int sys, const double *x, const double *xu, con
   CK(cudaStreamSynchronize(e->stream));  // host buffers may be freed on return
   e->hramp[sys] = 0;
   e->dirty[sys] = 1;
+  e->loaded[sys] = 1;
   e->any_dirty = true;
   return ACG_OK;
 }
@@ -1575,6 +1578,7 @@ int acg_set_lattice(acg_engine *e, int sys, const int *site, const int *type, co
   CK(cudaStreamSynchronize(e->stream));
   e->hramp[sys] = 0;
   e->dirty[sys] = 1;
+  e->loaded[sys] = 1;
   e->any_dirty = true;
   return ACG_OK;
 }
