@@ -390,30 +390,44 @@ __device__ __forceinline__ double nhc_link(double x, double &e) {
 // six exponentials, their divisions and the state in global memory a step took
 // 42.2 us at N = 1000 (FP64), 43.6 at N = 11154 (FP32), 95.8 at N = 100000;
 // with this form on the state in shared memory 39.0, 40.6 and 92.8.
-__device__ inline double nhc_half(double *eta, double *p_eta, const double *q, const double *rq, double T,
-                                  double dof, double dt, double ksum) {
+//
+// In two parts: what the half needs before the momenta's sum is known (links 2
+// and 1, the factors of 1 and 0), and the rest.
+// The fused multiply-adds are written out: both paths (the force kernels' last
+// block and k_run_box) have to round alike.
+struct NhcHalf {
+  double p1, p2, e1, f1, e0, f0;
+};
+__device__ __forceinline__ NhcHalf nhc_before(const double *p_eta, const double *rq, double T, double dt) {
   static_assert(NHC_M == 3, "the sweeps are written out for three links");
+  const double t4 = dt * 0.25;
+  NhcHalf h;
+  h.p2 = fma(t4, fma(p_eta[1] * p_eta[1], rq[1], -T), p_eta[2]);
+  h.f1 = nhc_link(t4 * h.p2 * rq[2], h.e1);
+  h.p1 = fma(p_eta[1], h.e1, t4 * fma(p_eta[0] * p_eta[0], rq[0], -T) * h.f1);
+  h.f0 = nhc_link(t4 * h.p1 * rq[1], h.e0);
+  return h;
+}
+__device__ __forceinline__ double nhc_after(const NhcHalf &h, double *eta, double *p_eta, const double *rq, double T,
+                                            double dof, double dt, double ksum) {
   const double t4 = dt * 0.25, t3 = dt * 0.50;
-  double p0 = p_eta[0], p1 = p_eta[1], p2 = p_eta[2];
-  p2 = p2 + t4 * ((p1 * p1) * rq[1] - T);
-  double e1, e0, es;
-  const double f1 = nhc_link(t4 * p2 * rq[2], e1);
-  p1 = p1 * e1 + t4 * ((p0 * p0) * rq[0] - T) * f1;
-  const double f0 = nhc_link(t4 * p1 * rq[1], e0);
-  p0 = p0 * e0 + t4 * (ksum - dof * T) * f0;
-  nhc_link(t3 * p0 * rq[0], es);
-  const double s = es;
-  eta[0] = eta[0] + t3 * p0 * rq[0];
-  eta[1] = eta[1] + t3 * p1 * rq[1];
-  eta[2] = eta[2] + t3 * p2 * rq[2];
+  double p0 = fma(p_eta[0], h.e0, t4 * fma(-dof, T, ksum) * h.f0);
+  double s;
+  nhc_link(t3 * p0 * rq[0], s);
+  eta[0] = fma(t3 * p0, rq[0], eta[0]);
+  eta[1] = fma(t3 * h.p1, rq[1], eta[1]);
+  eta[2] = fma(t3 * h.p2, rq[2], eta[2]);
   const double s2k = (s * s) * ksum;
-  p0 = p0 * e0 + t4 * (s2k - dof * T) * f0;
-  p1 = p1 * e1 + t4 * ((p0 * p0) * rq[0] - T) * f1;
-  p2 = p2 + t4 * ((p1 * p1) * rq[1] - T);
+  p0 = fma(p0, h.e0, t4 * fma(-dof, T, s2k) * h.f0);
+  const double p1 = fma(h.p1, h.e1, t4 * fma(p0 * p0, rq[0], -T) * h.f1);
+  p_eta[2] = fma(t4, fma(p1 * p1, rq[1], -T), h.p2);
   p_eta[0] = p0;
   p_eta[1] = p1;
-  p_eta[2] = p2;
   return s;
+}
+__device__ inline double nhc_half(double *eta, double *p_eta, const double *rq, double T, double dof, double dt,
+                                  double ksum) {
+  return nhc_after(nhc_before(p_eta, rq, T, dt), eta, p_eta, rq, T, dof, dt, ksum);
 }
 
 // Nose-Hoover NPT chains (MDcode/time_evolve.c:700-822).  U4PropagatorNPT:

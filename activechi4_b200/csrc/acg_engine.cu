@@ -355,24 +355,28 @@ RunFn run_fn(int tpp, int prec, int nt, bool resident) {
 
 // whether one system can run inside a cluster: whole-box lists from sub-cells,
 // an integrator whose step is a kick/drift and one force pass, no uniform
-// direction shuffle
+// direction shuffle.  (Systems of five and more cells per side, on the same
+// kernel with lists of their own: N = 4505 FP32 26 us a step against 34 kernel
+// by kernel, but N = 11154 60 against 38 -- 16 SMs against 148 -- and a line in
+// between would make a system's bits depend on the others of its engine.)
 bool run_eligible(const SysDesc &d) { return d.box && d.msub >= 5 && d.thermostat <= 2 && d.shuffle != 2; }
 
 // Cluster size, threads and shared memory of an engine's runs; run_c stays 0
 // where a system is not eligible or does not fit.  As many blocks per cluster
 // as leave every system its own cluster on the chip at once (7 of 16 blocks,
-// 15 of 8, 33 of 4, 74 of 2 with one block per SM), then one block per system.
+// 15 of 8, 33 of 4, 74 of 2 with one block per SM), then one block per system;
+// more where a system does not fit otherwise.
 void plan_run(acg_engine *e, size_t smem_limit) {
   const Layout &L = e->lay;
   e->run_c = 0;
   for (int r = 0; r < L.nsys; r++)
     if (!run_eligible(L.desc[r])) return;
-  const int C = L.nsys <= 7 ? 16 : (L.nsys <= 15 ? 8 : (L.nsys <= 33 ? 4 : (L.nsys <= 74 ? 2 : 1)));
+  const int C0 = L.nsys <= 7 ? 16 : (L.nsys <= 15 ? 8 : (L.nsys <= 33 ? 4 : (L.nsys <= 74 ? 2 : 1)));
   const int prec = L.desc[0].precision;
   // state in shared memory where it fits; threads per block: 512 (FP64 pair
   // terms take about 120 registers a thread), or 1024 for FP32 systems with
   // more slots per block than that
-  for (int resident = 1; resident >= 0; resident--) {
+  for (int C = C0, resident = 1; C <= 16; C = resident ? C : 2 * C, resident ^= 1) {
     int nloc = 0;
     for (const SysDesc &d : L.desc) nloc = std::max(nloc, 32 * (((d.n + 31) / 32 + C - 1) / C));
     const int nt = prec && !resident && nloc * 2 > 512 ? 1024 : 512;

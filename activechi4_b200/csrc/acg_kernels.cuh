@@ -1112,7 +1112,7 @@ __device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, Sys
       eta[k] = st.eta_end[k];
       pet[k] = st.p_eta_end[k];
     }
-    double s1 = nhc_half(eta, pet, d.q, d.rq, d.T, d.dof, d.dt, kb);
+    double s1 = nhc_half(eta, pet, d.rq, d.T, d.dof, d.dt, kb);
     for (int k = 0; k < NHC_M; k++) {
       st.eta_cur[k] = eta[k];
       st.p_eta_cur[k] = pet[k];
@@ -1243,7 +1243,7 @@ __device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, SysDe
         eta[k] = st.eta_cur[k];
         pet[k] = st.p_eta_cur[k];
       }
-      double s2 = nhc_half(eta, pet, d.q, d.rq, d.T, d.dof, d.dt, ke);
+      double s2 = nhc_half(eta, pet, d.rq, d.T, d.dof, d.dt, ke);
       for (int k = 0; k < NHC_M; k++) {
         st.eta_end[k] = eta[k];
         st.p_eta_end[k] = pet[k];
@@ -2864,25 +2864,27 @@ __device__ __forceinline__ void box_list_brick(const View &v, const SysDesc &d, 
   int nn = 0;          // entries moved to the list
   int u = 0;           // this lane's run
   __syncwarp();
-  for (int f0 = 0; f0 < Q; f0 += BRICK_BATCH) {
-    float4 c[BRICK_BATCH / 32];
-#pragma unroll
-    for (int e = 0; e < BRICK_BATCH / 32; e++) {
-      const int f = f0 + 32 * e + lane;
-      c[e] = make_float4(nan, nan, nan, __int_as_float(-1));
-      if (f < Q) {
-        while (S.first[u + 1] <= f) u++;
-        c[e] = xs[S.start[u] + (f - S.first[u])];
-        const int row = u / 3;
-        c[e].x += (float)(u - 3 * row - 1);
-        c[e].y += (float)S.sy[row];
-        c[e].z += (float)S.sz[row];
-      }
+  static_assert(BRICK_BATCH == 32, "one candidate a lane");
+  // candidate f0 + lane of the union, one batch ahead of the tests
+  auto fetch = [&](int f0) {
+    float4 c = make_float4(nan, nan, nan, __int_as_float(-1));
+    const int f = f0 + lane;
+    if (f < Q) {
+      while (S.first[u + 1] <= f) u++;
+      c = xs[S.start[u] + (f - S.first[u])];
+      const int row = u / 3;
+      c.x += (float)(u - 3 * row - 1);
+      c.y += (float)S.sy[row];
+      c.z += (float)S.sz[row];
     }
+    return c;
+  };
+  float4 next = fetch(0);
+  for (int f0 = 0; f0 < Q; f0 += BRICK_BATCH) {
     __syncwarp();
-#pragma unroll
-    for (int e = 0; e < BRICK_BATCH / 32; e++) S.cand[32 * e + lane] = c[e];
+    S.cand[lane] = next;
     __syncwarp();
+    next = fetch(f0 + BRICK_BATCH);
     // eight at a time: all their loads and distances before their appends (a
     // store to the column keeps later loads behind it)
 #pragma unroll 1
@@ -3309,6 +3311,7 @@ __device__ __forceinline__ PairAcc box_pairs(const View &v, const SysDesc &d, co
         const double xi = sx[sl], yi = sy[sl], zi = sz[sl];
         const PairParamsD P(ti, L);
         PairAcc bb = {0.0, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll 2
         for (int c = lane; c < nch; c += TPP) {
           const uint2 wn = c + TPP < nch ? lp[(size_t)(c + TPP) * stride] : make_uint2(0u, 0u);
           const int left = nn - 4 * c;

@@ -9,15 +9,18 @@
 //   * every block stages all positions in its shared memory (FP32: 32-bit fixed
 //     point, FP64: doubles) and owns a run of slots, whose state stays in its
 //     shared memory where that fits (else in L2);
-//   * kick/drift: each block moves its slots and stores the new positions into
-//     every block's staging (distributed shared memory), with its largest
-//     displacement; cluster barrier; every block takes the same rebuild decision;
+//   * kick/drift: each block moves its slots, writes the new positions as staged
+//     to memory and its largest displacement into every block (distributed
+//     shared memory); cluster barrier; every block takes the same rebuild
+//     decision and reads all positions (storing them into the other 15 blocks
+//     took 6400 cycles at N = 4000 FP64, this 2000: one read is wide and
+//     coalesced, the remote stores are neither);
 //   * forces from the lists (kept in shared memory where they fit), second half
 //     kick, sums per 32 slots stored into every block; cluster barrier; every
 //     block adds them up in the same order and runs the thermostat chain.
 //
-// Two cluster barriers a step and no global memory on the way, where the state
-// is resident.  Clusters are co-scheduled by the hardware and wait on nothing
+// Two cluster barriers and one exchange through L2 a step, where the state is
+// resident.  Clusters are co-scheduled by the hardware and wait on nothing
 // but their own barrier, so systems are independent: a batch runs one cluster
 // per system, largest first, and no system waits for another's rebuild.  A list
 // rebuild happens inside the cluster: every block sorts the system by cell (a
@@ -27,8 +30,8 @@
 //
 // What bounds it: the latency of a step's dependent phases for a lone system
 // (16 of 148 SMs busy), the issue rate of the pair terms for a batch.  Measured
-// on B200 against the kernel-by-kernel graphs: N = 1000 FP64 39.0 -> 15.1 us a
-// step, N = 4000 FP64 60 -> 38, 256 FP32 replicas 400 -> 245.
+// on B200 against the kernel-by-kernel graphs: N = 1000 FP64 39.0 -> 14.3 us a
+// step, N = 4000 FP64 60 -> 36, 256 FP32 replicas 400 -> 245.
 //
 // Sums, lists and particle order are those of the kernel-by-kernel step, so a
 // system's results are the same bits whichever path, cluster size or residency
@@ -238,6 +241,7 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
   __shared__ SysDesc sd;
   __shared__ double s_wmax[32], s_cmax[RUN_MAX_CLUSTER];
   __shared__ double s_obs[OBS_EMAX][OBS_NV];
+  __shared__ NhcHalf s_half;
   __shared__ int s_nnmax, s_brick;
   cg::cluster_group cl = cg::this_cluster();
   const int C = (int)cl.num_blocks(), rank = (int)cl.block_rank();
@@ -265,6 +269,9 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
   const RunState g = run_global(v), w = RES ? run_resident(rsm + P.state, P.nloc, v.kdir) : g;
   const int wb = RES ? -lo : poff;
   const uint2 *lists = reinterpret_cast<const uint2 *>(box_list(v, sd));
+  // the step's new positions as staged, for the other blocks (the download
+  // buffer, free while the system steps)
+  unsigned char *shared_pos = reinterpret_cast<unsigned char *>(v.stage_f + 3 * (size_t)poff);
   bool cached = false;
 
   // list lengths of the block's slots, and their lists where they fit in the cache
@@ -307,8 +314,8 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
   bar();  // every block of the cluster runs and is staged
 
   for (int it = 0; it < nsteps; it++) {
-    // ---- kick and drift of the block's slots
     const bool shuf = tau && ramp == 0 && shuf_at == 0;
+    // ---- kick and drift of the block's slots
     if (tid == 0) {
       ss.shuf = shuf;
       ss.drift = sd.drift_every > 0 && ramp == 0 && drift_at == 0;
@@ -322,26 +329,13 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
     for (int k = lo + tid; k < hi; k += NT) {
       far = fmax(far, kick_drift_one(w, sd, ss, wb + k));
       const double4 p = w.pos[wb + k];
-      run_stage<PREC>(stg, n, k, p);
+      run_stage<PREC>(C > 1 ? shared_pos : stg, n, k, p);
       if (ovf && RES) v.pos[poff + k] = p;
     }
     for (int o = 16; o > 0; o >>= 1) far = fmax(far, __shfl_xor_sync(0xffffffffu, far, o));
     if (lane == 0) s_wmax[warp] = far;
     __syncthreads();
-    // the new positions and the largest displacement to every block
-    for (int q = tid; q < own * (C - 1); q += NT) {
-      const int c = q / own, k = lo + q - c * own;
-      unsigned char *there = cl.map_shared_rank(stg, (rank + 1 + c) % C);
-      if (PREC == 1) {
-        const int *a = reinterpret_cast<const int *>(stg);
-        int *b = reinterpret_cast<int *>(there);
-        for (int x = 0; x < 3; x++) b[x * n + k] = a[x * n + k];
-      } else {
-        const double *a = reinterpret_cast<const double *>(stg);
-        double *b = reinterpret_cast<double *>(there);
-        for (int x = 0; x < 3; x++) b[x * n + k] = a[x * n + k];
-      }
-    }
+    // the largest displacement to every block
     if (warp == 0) {
       far = lane < NW ? s_wmax[lane] : 0.0;
       for (int o = 16; o > 0; o >>= 1) far = fmax(far, __shfl_xor_sync(0xffffffffu, far, o));
@@ -359,9 +353,20 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
       ss.rebuild = rebuild;
       ss.force_rebuild = 0;
     }
+    if (!rebuild && C > 1) {  // every block's new positions
+      const uint4 *from = reinterpret_cast<const uint4 *>(shared_pos);
+      uint4 *to = reinterpret_cast<uint4 *>(stg);
+      const int words = 3 * n * (PREC ? 4 : 8) / 4;
+      for (int q = tid; q < words / 4; q += NT) to[q] = __ldcg(from + q);
+      if (tid < words % 4)
+        reinterpret_cast<unsigned *>(stg)[words / 4 * 4 + tid] =
+            __ldcg(reinterpret_cast<const unsigned *>(shared_pos) + words / 4 * 4 + tid);
+      __syncthreads();
+    }
     if (rebuild) {
       const int m3 = sd.msub * sd.msub * sd.msub;
       float4 *xs = reinterpret_cast<float4 *>(stg);
+      uint16_t *hist = reinterpret_cast<uint16_t *>(stg);
       int *sst = reinterpret_cast<int *>(stg + P.lists_at - run_align(4 * (size_t)(m3 + 1)));
       uint16_t *key = reinterpret_cast<uint16_t *>(stg + P.lists_at);
       uint16_t *ord = reinterpret_cast<uint16_t *>(stg + P.lists_at + run_align(2 * (size_t)n));
@@ -376,8 +381,7 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
         if (rank == 0) v.st[r].overflow = 0;
       }
       bar();
-      run_sort_cells(v, sd, perm, key, ord, reinterpret_cast<uint16_t *>(xs),
-                     reinterpret_cast<int *>(reinterpret_cast<uint16_t *>(xs) + (size_t)NW * sd.ncell), rank == 0);
+      run_sort_cells(v, sd, perm, key, ord, hist, reinterpret_cast<int *>(hist + (size_t)NW * sd.ncell), rank == 0);
       if (RES) {
         for (int k = lo + tid; k < hi; k += NT) {
           run_copy_slot(w, wb + k, g, poff + perm[k]);
@@ -461,6 +465,8 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
       if (tid < nev && (ob.ev_info[ob_lo + tid] & 1) == 0) obs_accumulate(ob, n, ob.ev_info[ob_lo + tid], s_obs[tid]);
     }
     // ---- forces, second half kick, sums per 8 and per 32 slots
+    const bool nose = sd.thermostat == 1 && ramp == 0;
+    if (nose && tid == NT - 32) s_half = nhc_before(ss.p_eta_cur, sd.rq, sd.T, sd.dt);
     for (int b = warp * (32 / TPP); b < 32 * nseg_own; b += NT / TPP) {
       const int k = b + lane / TPP;
       const bool valid = k < own;
@@ -480,8 +486,51 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
       *cl.map_shared_rank(&seg[lo_seg + q % nseg_own], q / nseg_own) = add4(add4(s8[0], s8[1]), add4(s8[2], s8[3]));
     }
     bar();
-    // ---- system sums and thermostat, the same in every block
-    if (warp == 0) {
+    // ---- system sums and thermostat, the same in every block.  A Nose-Hoover
+    // step's chain, the longest chain of dependent operations of a small system's
+    // step, is one warp's, the part of it that needs no sums computed beforehand
+    // by another; a third adds up the energies (finalize_sums' operations)
+    if (nose) {
+      if (warp == 0) {
+        double k2 = 0.0;
+        for (int q = lane; q < P.nseg; q += 32) k2 += seg[q].z;
+        for (int o = 16; o > 0; o >>= 1) k2 += __shfl_xor_sync(0xffffffffu, k2, o);
+        if (lane == 0) {
+          double eta[NHC_M], pet[NHC_M];
+          for (int k = 0; k < NHC_M; k++) {
+            eta[k] = ss.eta_cur[k];
+            pet[k] = ss.p_eta_cur[k];
+          }
+          const double s2 = nhc_after(s_half, eta, pet, sd.rq, sd.T, sd.dof, sd.dt, k2);
+          const double kb = (s2 * s2) * k2;
+          for (int k = 0; k < NHC_M; k++) {
+            ss.eta_end[k] = eta[k];
+            ss.p_eta_end[k] = pet[k];
+          }
+          ss.s1 = nhc_half(eta, pet, sd.rq, sd.T, sd.dof, sd.dt, kb);
+          ss.s2 = s2;
+          for (int k = 0; k < NHC_M; k++) {
+            ss.eta_cur[k] = eta[k];
+            ss.p_eta_cur[k] = pet[k];
+          }
+          ss.ke_end = kb * 0.5;
+          if (!(k2 == k2) || k2 > 1.0e300) ss.status = 1;
+        }
+      } else if (warp == 1) {
+        double4 t = total_of_segments(seg, P.nseg);
+        if (lane == 0) {
+          ss.pe = 0.5 * t.x;
+          ss.virial = (0.5 * t.y) / 3.0;
+          ss.vir_act = t.w;
+          ss.step += 1;
+          if (shuf) {
+            ss.mt_cur ^= 1;
+            ss.shuf = 0;
+          }
+          ss.prime = 0;
+        }
+      }
+    } else if (warp == 0) {
       const double4 t = total_of_segments(seg, P.nseg);
       if (lane == 0) finalize_sums(sd, ss, sd, 0, t.x, t.y, t.z, t.w);
     }
