@@ -73,7 +73,7 @@ constexpr int MAX_BOX_N = 8192;   // whole-box staging limit (FP64: 192 KB of sh
 constexpr int MAX_SUB3 = 1000;    // list sub-cells of a whole box (side >= 1.45 and L < 15: <= 10^3)
 constexpr int MT_N = 624;         // MT19937 state words
 constexpr int MT_WORDS = 625;     // one stored state: 624 words + the next word's index
-constexpr int BLOCK_SHUF = 256;   // threads of the reference-order direction shuffle
+constexpr int BLOCK_SHUF = 640;   // threads of the reference-order direction shuffle (a swap of 624 draws each)
 constexpr int SHUF_SMEM_NACT = 32768;  // directions staged in shared memory up to this many
 
 // A cell group: up to 2 x 2 x 2 cells (clipped at the box edge) and the union

@@ -321,8 +321,11 @@ size_t box_smem(int nmax, int prec) { return (size_t)nmax * 3 * (prec ? sizeof(i
 // 16-bit arrays of n and the sub-cell starts and counters.
 size_t box_list_smem_cells(int nmax) { return ((size_t)nmax + 3 * MAX_BOX_CELLS) * sizeof(float4); }
 size_t box_list_smem(int cell_nmax) { return cell_nmax > 0 ? box_list_smem_cells(cell_nmax) : 0; }
-// reference-order shuffle: one system's directions staged as bytes
-size_t shuffle_smem(const Layout &lay) { return align_up((size_t)std::max(1, std::min(lay.nact_max, SHUF_SMEM_NACT)), 16); }
+// reference-order shuffle: one system's directions staged as bytes, a mark for each
+size_t shuffle_smem(const Layout &lay) {
+  const size_t a = (size_t)std::max(1, std::min(lay.nact_max, SHUF_SMEM_NACT));
+  return align_up(a, 16) + align_up(4 * a, 16);
+}
 size_t sort_sub_smem(int nmax, int m3max) { return (size_t)nmax * 2 * sizeof(uint16_t) + (2 * (size_t)m3max + 1) * sizeof(int); }
 
 ForceFn force_fn(int tpp, int prec) {
@@ -687,7 +690,7 @@ int launch_step_eager(acg_engine *e) {
   int rc0 = launch_pre(e);
   if (rc0) return rc0;
   k_kick_drift<<<e->ntiles_a + 3 * e->lay.nsys, BLOCK_A, 0, e->stream>>>(e->v, 0, 0);
-  k_shuffle_ref<<<3 * e->lay.nsys, BLOCK_SHUF, shuffle_smem(e->lay), e->stream>>>(e->v, -1);
+  k_shuffle_ref<<<3 * e->lay.nsys, BLOCK_SHUF, shuffle_smem(e->lay), e->stream>>>(e->v, -1, (int)shuffle_smem(e->lay));
   CK(cudaGetLastError());
   int rc = launch_rebuild(e);
   if (rc) return rc;
@@ -820,8 +823,8 @@ int add_steps(acg_engine *e, cudaGraph_t g, int K, cudaGraphNode_t *prev_io) {
               {(void *)k_build_list_box, e->ntiles_x * LIST_SPLIT, BLOCK_X, box_list_smem(e->lay.box_cell_nmax)},
               {(void *)k_build_list_cells, e->ntiles_lc, BLOCK_LC, list_cells_smem(v.lccap)},
               {(void *)k_build_list, e->ntiles_l, BLOCK_L, 0}};
-    int all = -1;
-    void *sa[] = {&v, &all};
+    int all = -1, sbytes = (int)shuffle_smem(e->lay);
+    void *sa[] = {&v, &all, &sbytes};
     for (int c = 0; c < 7; c++) {
       const int bits = c + 1;
       cudaGraph_t body = cp.conditional.phGraph_out[c];
@@ -1210,6 +1213,7 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
   }
   for (int gt : {1, 2, 4})
     for (int pr : {0, 1}) attr_ok = attr_ok && raise_smem((const void *)group_fn(gt, pr), group_smem(v.gcap));
+  attr_ok = attr_ok && raise_smem((const void *)k_shuffle_ref, shuffle_smem(L));
   attr_ok = attr_ok && raise_smem((const void *)k_build_list_groups, list_smem(v.gcap));
   attr_ok = attr_ok && raise_smem((const void *)k_build_list_cells, list_cells_smem(v.lccap));
   if (L.box_nmax > 0) {
@@ -1444,7 +1448,7 @@ int acg_shuffle_directions(acg_engine *e, int sys) {
   if (e->lay.desc[sys].shuffle == 2) {
     k_shuffle_now<<<3, 256, 0, e->stream>>>(e->v, sys);
   } else {
-    k_shuffle_ref<<<3, BLOCK_SHUF, shuffle_smem(e->lay), e->stream>>>(e->v, sys);
+    k_shuffle_ref<<<3, BLOCK_SHUF, shuffle_smem(e->lay), e->stream>>>(e->v, sys, (int)shuffle_smem(e->lay));
     k_mt_flip<<<1, 32, 0, e->stream>>>(e->v, sys);
   }
   CK(cudaGetLastError());

@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
       for (int c = 0; c < 3; c++)
         if (c % C == rank) {
           shuffle_ref_component(v, r, c, mt + (size_t)ss.mt_cur * MT_WORDS, mt + (size_t)(ss.mt_cur ^ 1) * MT_WORDS,
-                                reinterpret_cast<signed char *>(rsm));
+                                reinterpret_cast<signed char *>(rsm), P.seg8);
           __syncthreads();
         }
     }
