@@ -2059,10 +2059,6 @@ __device__ __forceinline__ size_t group_entry(int k, int t, int M) {
   return ((size_t)(k >> 2) * M + t) * 4 + (k & 3);
 }
 
-// 16-bit list entries of one particle, packed four to a chunk in a 64-bit
-// shift register (the newest entry enters at the top, so after four the
-// first is in the low bits); whole chunks are stored as uint2 at
-// chunk * stride + row
 // the next index of a block-shared counter for the calling warp (lane 0 takes
 // it, the warp shares it)
 __device__ __forceinline__ int warp_next(int &counter) {
@@ -2071,23 +2067,57 @@ __device__ __forceinline__ int warp_next(int &counter) {
   return __shfl_sync(0xffffffffu, o, 0);
 }
 
-struct ListWriter {
-  unsigned lo = 0u, hi = 0u;
-  int n = 0;
-  __device__ __forceinline__ void add(unsigned code, uint2 *lst, size_t stride, int row, int maxnb) {
-    lo = __funnelshift_r(lo, hi, 16);
-    hi = (hi >> 16) | (code << 16);
-    n++;
-    if ((n & 3) == 0 && n <= maxnb) lst[(size_t)((n >> 2) - 1) * stride + row] = make_uint2(lo, hi);
+// A lane's column of accepted candidates in shared memory (entries 64 bytes
+// apart: 32 lanes of 16-bit codes): a candidate within the cut and not the
+// particle itself is appended by a predicated store and a pointer step, not a
+// branch (with 32 lanes nearly every candidate is accepted by one of them, so all
+// would pay for the append)
+constexpr int COLUMN_ROWS = 36;  // 32 candidates between two flushes and three left over
+struct ListColumn {
+  uint16_t *col;
+  unsigned first, at;  // shared-memory address of the column and of its next free entry
+  int n = 0;           // entries moved to the list
+  __device__ __forceinline__ explicit ListColumn(uint16_t *c)
+      : col(c), first((unsigned)__cvta_generic_to_shared(c)), at(first) {}
+  __device__ __forceinline__ void test(float r2, float cut, int code, int self) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.lt.f32 p, %1, %2;\n\t"
+        "setp.ne.and.s32 p, %3, %4, p;\n\t"
+        "@p st.shared.u16 [%0], %5;\n\t"
+        "@p add.u32 %0, %0, 64;\n\t}"
+        : "+r"(at)
+        : "f"(r2), "f"(cut), "r"(code), "r"(self), "h"((unsigned short)code)
+        : "memory");
   }
-  // the last, partial chunk: its k pending entries sit in the top 16k bits
-  __device__ __forceinline__ void finish(uint2 *lst, size_t stride, int row, int maxnb, unsigned pad = 0u) {
-    const int k = n & 3;
-    if (k && n <= maxnb) {
-      unsigned long long p = (((unsigned long long)hi << 32) | lo) >> (16 * (4 - k));
-      for (int e = k; e < 4; e++) p |= (unsigned long long)pad << (16 * e);
-      lst[(size_t)(n >> 2) * stride + row] = make_uint2((unsigned)p, (unsigned)(p >> 32));
+  // full chunks of four to the list (chunk c at lst[c * stride + row]), the
+  // rest to the front of the column
+  __device__ __forceinline__ void flush(uint2 *lst, size_t stride, int row, int maxnb) {
+    int from = 0;
+    for (; (int)(at - first) - 2 * from >= 256; from += 128) {
+      if (n + 4 <= maxnb)
+        lst[(size_t)(n >> 2) * stride + row] =
+            make_uint2(col[from] | ((unsigned)col[from + 32] << 16), col[from + 64] | ((unsigned)col[from + 96] << 16));
+      n += 4;
     }
+    if (from) {
+      const uint16_t a0 = col[from], a1 = col[from + 32], a2 = col[from + 64];
+      col[0] = a0;
+      col[32] = a1;
+      col[64] = a2;
+      at -= 2 * from;
+    }
+  }
+  // the last, partial chunk, padded with `pad` (< 0: its last entry)
+  __device__ __forceinline__ void finish(uint2 *lst, size_t stride, int row, int maxnb, int pad) {
+    const int left = (int)(at - first) >> 6;
+    if (left && n + left <= maxnb) {
+      const unsigned e0 = col[0], e1 = left > 1 ? col[32] : (pad < 0 ? e0 : (unsigned)pad),
+                     e2 = left > 2 ? col[64] : (pad < 0 ? e1 : (unsigned)pad),
+                     e3 = pad < 0 ? e2 : (unsigned)pad;
+      lst[(size_t)(n >> 2) * stride + row] = make_uint2(e0 | (e1 << 16), e2 | (e3 << 16));
+    }
+    n += left;
   }
 };
 
@@ -2151,6 +2181,7 @@ __global__ void __launch_bounds__(BLOCK_G) k_build_list_groups(View v) {
   __shared__ GroupStage S;
   __shared__ int pre4[MAX_UNION + 1];
   __shared__ int s_over;  // next overflow particle to hand out
+  __shared__ uint16_t s_col[BLOCK_G / 32][COLUMN_ROWS][32];
   const int2 tile = v.tiles_g[blockIdx.x];
   const int r = tile.x;
   if (!v.st[r].rebuild) return;
@@ -2233,12 +2264,12 @@ __global__ void __launch_bounds__(BLOCK_G) k_build_list_groups(View v) {
     } else {
       // an unsplit group (many groups per system): one warp per centre cell,
       // one lane per particle, every lane testing the same staged candidate
-      // (a shared-memory broadcast); each lane packs its entries into a 64-bit
-      // register and stores whole 4-entry chunks (the same lists: cells in
-      // (dz, dy, dx) order, staged order inside a cell)
+      // (a shared-memory broadcast) and appending to its column (the same lists:
+      // cells in (dz, dy, dx) order, staged order inside a cell).  With the
+      // append in registers behind a branch a rebuild took 165 us at N = 100000
+      // and 341 us at N = 256000 (FP64)
       float lc[3];
       for (int k = 0; k < 3; k++) lc[k] = (float)(lcut2_of(d, k) * (1.0 + 1e-5));
-      const bool one_cut = lc[0] == lc[1] && lc[1] == lc[2];
       uint2 *lst = reinterpret_cast<uint2 *>(group_list(v, d, g));
       // the first 32 particles of each centre cell; a cell's further
       // particles (a dense cell) are listed below, one warp each, so that no
@@ -2251,36 +2282,40 @@ __global__ void __launch_bounds__(BLOCK_G) k_build_list_groups(View v) {
           const int w = lane;
           const bool valid = w < m;
           const int t = S.cpre[kc] + w, ps = pre4[cu] + w;
-          const float4 fi = valid ? stg[ps] : make_float4(-1e18f, -1e18f, -1e18f, __int_as_float(0));
+          // a lane past the cell's particles: NaN coordinates pass no test
+          const float nan = __int_as_float(0x7fc00000);
+          const float4 fi = valid ? stg[ps] : make_float4(nan, nan, nan, __int_as_float(0));
           const int ti = __float_as_int(fi.w) >> 15;
           // cut for a partner of type 0 / 1 (the sum of the two types indexes lc)
           const float c0 = ti == 0 ? lc[0] : lc[1], c1 = ti == 0 ? lc[1] : lc[2];
-          ListWriter lw;
+          const int codei = valid ? __float_as_int(fi.w) : -1;
+          ListColumn col(&s_col[warp][0][lane]);
           for (int dz = -1; dz <= 1; dz++)
             for (int dy = -1; dy <= 1; dy++)
               for (int dx = -1; dx <= 1; dx++) {
                 const int u2 = (ux + dx) + (uy + dy) * nux + (uz + dz) * nux * nuy;
                 const int q1 = pre4[u2 + 1];
-                for (int q = pre4[u2]; q < q1; q += 4) {
-                  int code[4];
-                  bool ok[4];
+                for (int q0 = pre4[u2]; q0 < q1; q0 += 32) {
+#pragma unroll 1
+                  for (int q = q0; q < min(q1, q0 + 32); q += 4) {
+                    float r2[4];
+                    int code[4];
 #pragma unroll
-                  for (int e = 0; e < 4; e++) {
-                    const float4 fj = stg[q + e];
-                    const float ex = fi.x - fj.x, ey = fi.y - fj.y, ez = fi.z - fj.z;
-                    const float r2 = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
-                    code[e] = __float_as_int(fj.w);
-                    const float cut = one_cut ? c0 : ((code[e] >> 15) ? c1 : c0);
-                    ok[e] = valid && r2 < cut && q + e != ps;
+                    for (int e = 0; e < 4; e++) {
+                      const float4 fj = stg[q + e];
+                      const float ex = fi.x - fj.x, ey = fi.y - fj.y, ez = fi.z - fj.z;
+                      r2[e] = fmaf(ex, ex, fmaf(ey, ey, ez * ez));
+                      code[e] = __float_as_int(fj.w);
+                    }
+#pragma unroll
+                    for (int e = 0; e < 4; e++) col.test(r2[e], code[e] > 0x7fff ? c1 : c0, code[e], codei);
                   }
-#pragma unroll
-                  for (int e = 0; e < 4; e++)
-                    if (ok[e]) lw.add((unsigned)code[e] & 0xffffu, lst, M, t, maxnb);
+                  col.flush(lst, M, t, maxnb);
                 }
               }
           if (valid) {
-            lw.finish(lst, M, t, maxnb, (unsigned)v.gcap);
-            const int n = lw.n;
+            col.finish(lst, M, t, maxnb, v.gcap);
+            const int n = col.n;
             const int i = S.ustart[cu] + w;
             if (n > maxnb) {
               v.nbn[i] = -1;
@@ -2817,7 +2852,7 @@ constexpr int BRICK_ROWS = 36;  // (z, y) rows of a union at most (2 x 2 x 2 bri
 constexpr int BRICK_BATCH = 32;
 struct BrickScratch {           // one warp's shared memory
   float4 cand[BRICK_BATCH];
-  uint16_t col[BRICK_BATCH + 4][32];  // a batch's entries and three left over per lane
+  uint16_t col[COLUMN_ROWS][32];  // the lanes' columns
   uint16_t start[3 * BRICK_ROWS], first[3 * BRICK_ROWS + 4];  // runs: start in sub-cell order, candidates before
   signed char sy[BRICK_ROWS], sz[BRICK_ROWS];                 // image of each row
 };
@@ -2892,11 +2927,8 @@ __device__ __forceinline__ void box_list_brick(const View &v, const SysDesc &d, 
   const int sl = codei & 0x7fff;
   float c0, c1;
   box_cuts(d, valid ? codei >> 15 : 0, c0, c1);
-  const uint16_t *const col = &S.col[0][lane];
-  const unsigned col0 = (unsigned)__cvta_generic_to_shared(col);
-  unsigned at = col0;  // the column's next free entry (entries 64 bytes apart)
-  int nn = 0;          // entries moved to the list
-  int u = 0;           // this lane's run
+  ListColumn col(&S.col[0][lane]);
+  int u = 0;  // this lane's run
   __syncwarp();
   static_assert(BRICK_BATCH == 32, "one candidate a lane");
   // candidate f0 + lane of the union, one batch ahead of the tests
@@ -2933,48 +2965,18 @@ __device__ __forceinline__ void box_list_brick(const View &v, const SysDesc &d, 
         code[e] = __float_as_int(fj.w);
       }
 #pragma unroll
-      for (int e = 0; e < 8; e++)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.lt.f32 p, %1, %2;\n\t"
-            "setp.ne.and.s32 p, %3, %4, p;\n\t"
-            "@p st.shared.u16 [%0], %5;\n\t"
-            "@p add.u32 %0, %0, 64;\n\t}"
-            : "+r"(at)
-            : "f"(r2[e]), "f"(code[e] > 0x7fff ? c1 : c0), "r"(code[e]), "r"(codei), "h"((unsigned short)code[e])
-            : "memory");
+      for (int e = 0; e < 8; e++) col.test(r2[e], code[e] > 0x7fff ? c1 : c0, code[e], codei);
     }
-    // full chunks to the list, the rest to the front of the column
-    int from = 0;
-    for (; (int)(at - col0) - 2 * from >= 256; from += 128) {
-      if (nn + 4 <= maxnb)
-        lst[(size_t)(nn >> 2) * n + sl] =
-            make_uint2(col[from] | ((unsigned)col[from + 32] << 16), col[from + 64] | ((unsigned)col[from + 96] << 16));
-      nn += 4;
-    }
-    if (from) {
-      const uint16_t a0 = col[from], a1 = col[from + 32], a2 = col[from + 64];
-      uint16_t *const front = &S.col[0][lane];
-      front[0] = a0;
-      front[32] = a1;
-      front[64] = a2;
-      at -= 2 * from;
-    }
+    col.flush(lst, n, sl, maxnb);
   }
   if (valid) {
-    // the last, partial chunk, padded with its last entry
-    const int left = (int)(at - col0) >> 6;
-    if (left && nn + left <= maxnb) {
-      const unsigned e0 = col[0], e1 = left > 1 ? col[32] : e0, e2 = left > 2 ? col[64] : e1;
-      lst[(size_t)(nn >> 2) * n + sl] = make_uint2(e0 | (e1 << 16), e2 | (e2 << 16));
-    }
-    nn += left;
+    col.finish(lst, n, sl, maxnb, -1);
     const int i = d.poff + sl;
-    if (nn > maxnb) {
+    if (col.n > maxnb) {
       v.nbn[i] = -1;
       atomicAdd(&v.st[r].overflow, 1);
     } else {
-      v.nbn[i] = nn;
+      v.nbn[i] = col.n;
     }
   }
   __syncwarp();
