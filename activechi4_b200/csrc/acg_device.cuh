@@ -45,7 +45,10 @@ constexpr int LIST_SPLIT = 4;     // blocks sharing a whole-box tile in the list
 #define ACG_BRICK2_MAX 28.0
 #endif
 constexpr double BRICK2_MAX = ACG_BRICK2_MAX;
-constexpr int BOX_WARP_MAX = 16384;  // whole-box particles up to which lists are built one warp per particle
+// whole-box particles up to which the list kernel builds lists one warp per
+// particle (rebuild, us, per particle / by bricks: N = 1000 78 / 88, N = 2000 104
+// / 88, N = 4000 99 / 98)
+constexpr int BOX_WARP_MAX = 1500;
 constexpr int GSPLIT_MAX = 8;     // most force blocks per cell group (small boxes)
 // measured on B200 (FP32, T = 0.45, step latency of one system alone):
 // N = 4505 43-47 us per step on the per-particle kernels against 53 us on

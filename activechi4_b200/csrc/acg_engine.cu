@@ -401,19 +401,24 @@ void plan_run(acg_engine *e, size_t smem_limit) {
   }
 }
 
-// nsteps steps of every system, one cluster each
-int launch_run(acg_engine *e, int nsteps) {
-  cudaLaunchConfig_t cfg = {};
+void run_config(const acg_engine *e, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
+  cfg = {};
   cfg.gridDim = dim3(e->lay.nsys * e->run_c);
   cfg.blockDim = dim3(e->run_nt);
   cfg.dynamicSmemBytes = e->run_smem;
   cfg.stream = e->stream;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = e->run_c;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-  cfg.attrs = at;
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = e->run_c;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
   cfg.numAttrs = 1;
+}
+
+// nsteps steps of every system, one cluster each
+int launch_run(acg_engine *e, int nsteps) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute at;
+  run_config(e, cfg, at);
   CK(cudaLaunchKernelEx(&cfg, run_fn(e->btpp, e->lay.desc[0].precision, e->run_nt, e->run_resident), e->v,
                         (const int *)e->run_order, nsteps, (unsigned)e->run_smem));
   return ACG_OK;
@@ -1206,9 +1211,19 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
     run_order.swap(ord);
     for (int gt : {1, 2, 4}) {
       const void *fn = (const void *)run_fn(gt, L.desc[0].precision, e->run_nt, e->run_resident);
-      attr_ok = attr_ok && raise_smem(fn, e->run_smem);
-      if (e->run_c > 8)
-        attr_ok = attr_ok && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      bool ok = raise_smem(fn, e->run_smem);
+      if (ok && e->run_c > 8)
+        ok = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+      // a device (or a part of one) that cannot hold such a cluster steps kernel by kernel
+      int clusters = 0;
+      cudaLaunchConfig_t cfg;
+      cudaLaunchAttribute at;
+      run_config(e, cfg, at);
+      if (!ok || cudaOccupancyMaxActiveClusters(&clusters, fn, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        e->run_c = 0;
+        break;
+      }
     }
   }
   for (int gt : {1, 2, 4})

@@ -239,7 +239,9 @@ int acg_compute_forces(acg_engine *e);
  * when due (MDcode/main.c:245-247) then AdvanceTimeNVTNoseHoover
  * (MDcode/time_evolve.c:495-526) or advance_time_NVEFrog
  * (MDcode/time_evolve.c:104-171).  Runs as CUDA-graph launches on the
- * engine's stream; returns after queuing (acg_sync waits). */
+ * engine's stream, or, where every system has 2 to 4 cells per side, as one
+ * kernel that advances each system inside a thread-block cluster; returns after
+ * queuing (acg_sync waits). */
 int acg_step(acg_engine *e, int nsteps);
 /* The same steps launched kernel by kernel without a CUDA graph (every
  * rebuild kernel is launched and skips the systems that need no rebuild). */
@@ -308,7 +310,8 @@ int acg_time_stage(acg_engine *e, int stage, int reps, double *ms);
 
 /* Benchmark timing: advance every system exactly nsteps steps as CUDA-graph
  * launches (one graph of nsteps steps up to 256, else graphs of 32 steps and
- * one of the remainder), recording CUDA events on the engine stream around
+ * one of the remainder; cluster runs: one kernel in place of each graph),
+ * recording CUDA events on the engine stream around
  * each launch, and write flush_bytes (> L2) with cudaMemsetAsync before each
  * launch (untimed) so that every timed launch starts from a cold L2.  *ms =
  * summed device time of the launches; *launches = kernels launched inside
