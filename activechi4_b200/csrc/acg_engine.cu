@@ -1290,6 +1290,8 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
   }
   rc = build_tiles_b(e);
   if (rc) return cleanup_fail(rc);
+  k_blank<<<e->ntiles_a, BLOCK_A, 0, e->stream>>>(e->v);
+  if (cudaGetLastError() != cudaSuccess) return cleanup_fail(fail(ACG_ERR_CUDA, "initial slots failed"));
   e->dirty.assign(nsys, 1);
   e->loaded.assign(nsys, 0);
   e->hstep.assign(nsys, 0);

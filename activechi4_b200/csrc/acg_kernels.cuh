@@ -3442,6 +3442,19 @@ __global__ void k_set_count(long long *count, long long n) {
 
 // ---------------------------------------------------------------------------
 // state upload / download (caller order <-> slots)
+
+// slots of systems that hold no state yet: particle k in slot k, none active.
+// The sorts take `id` as a permutation of a system's particles, and an
+// unloaded system steps with the others, at rest whatever its directions.
+__global__ void __launch_bounds__(BLOCK_A) k_blank(View v) {
+  const int2 t = v.tiles_a[blockIdx.x];
+  const SysDesc &d = v.desc[t.x];
+  const int k = t.y + threadIdx.x;
+  if (k >= d.n) return;
+  v.id[d.poff + k] = k;
+  v.act[d.poff + k] = -1;
+}
+
 __global__ void k_load(View v, int r) {
   const SysDesc &d = v.desc[r];
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < d.n; k += gridDim.x * blockDim.x) {
