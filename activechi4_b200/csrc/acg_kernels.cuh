@@ -515,16 +515,19 @@ __device__ __forceinline__ void obs_particle(const ObsDesc &o, int n, int info, 
   if (mz >= 0.5) mz -= 1.0; else if (mz < -0.5) mz += 1.0;
   if (my >= 0.5) my -= 1.0; else if (my < -0.5) my += 1.0;
   if (mx >= 0.5) mx -= 1.0; else if (mx < -0.5) mx += 1.0;
-  const double r2q = L * L * (mx * mx + my * my + mz * mz);
+  // every multiply-add is written out: k_observe and k_run_box have to round alike
+  const double L2 = L * L, x2 = dx * dx, y2 = dy * dy, z2 = dz * dz;
+  const double r2q = L2 * fma(mx, mx, fma(my, my, mz * mz));
   val[0] = r2q < o.a2 ? 1.0 : 0.0;
-  const double r2 = L * L * (dx * dx + dy * dy + dz * dz);
+  const double r2 = L2 * __dadd_rn(__dadd_rn(x2, y2), z2);
   val[1] = r2;
-  val[2] = L * L * L * L * (dx * dx * dx * dx + dy * dy * dy * dy + dz * dz * dz * dz);
-  val[3] = r2 * r2;
+  val[2] = (L2 * L2) * fma(x2, x2, fma(y2, y2, __dmul_rn(z2, z2)));
+  val[3] = __dmul_rn(r2, r2);
   double fs = 0.0;
   for (int q = 0; q < o.nq; q++)
-    fs += cos(6.283185307179586 * ((double)o.qvec[3 * q] * dx + (double)o.qvec[3 * q + 1] * dy +
-                                   (double)o.qvec[3 * q + 2] * dz));
+    fs = __dadd_rn(fs, cos(6.283185307179586 * fma((double)o.qvec[3 * q], dx,
+                                                   fma((double)o.qvec[3 * q + 1], dy,
+                                                       __dmul_rn((double)o.qvec[3 * q + 2], dz)))));
   val[4] = fs;
 }
 
@@ -535,7 +538,7 @@ __device__ __forceinline__ void obs_accumulate(const ObsDesc &o, int n, int info
   const double Q = sum[0] / tot;
   double *acc = o.acc + (size_t)bin * 8;
   acc[0] += Q;  // c[time_index] (Analysis/overlap.c:90-93)
-  acc[1] += Q * Q;
+  acc[1] = fma(Q, Q, acc[1]);
   acc[2] += sum[1] / tot;  // msd[0..2] (Analysis/msd_pos.c:88-91)
   acc[3] += sum[2] / tot;
   acc[4] += sum[3] / tot;
@@ -993,12 +996,13 @@ __global__ void __launch_bounds__(BLOCK_L) k_build_list(View v) {
 // ---------------------------------------------------------------------------
 // pair term (MDcode/cell_list+forces.c:174-203).  dr2/sigma^2 and 1/dr2 use
 // the precomputed 1/sigma^2 instead of the reference's two divisions; the
-// results agree to rounding.
+// results agree to rounding.  The multiply-adds are written out, so a kernel's
+// rounding does not depend on what the compiler contracts there.
 __device__ __forceinline__ void pair_fp64(PairAcc &a, const double4 &pi, int ti, const double4 &pj,
                                           double L, double L2) {
   const int tp = ti + (int)pj.w;
   double dx = min_image(pi.x - pj.x), dy = min_image(pi.y - pj.y), dz = min_image(pi.z - pj.z);
-  double dr2 = (dx * dx + dy * dy + dz * dz) * L2;
+  double dr2 = fma(dx, dx, fma(dy, dy, dz * dz)) * L2;
   // 1/sigma^2, 4 eps, 8 eps/sigma^2 for AA / AB / BB
   const double is2 = tp == 0 ? 1.0 : (tp == 1 ? 1.5625 : 1.0 / (0.88 * 0.88));
   double rs2 = dr2 * is2;
@@ -1006,13 +1010,13 @@ __device__ __forceinline__ void pair_fp64(PairAcc &a, const double4 &pi, int ti,
     const double e4 = tp == 0 ? 4.0 : (tp == 1 ? 6.0 : 2.0);
     double s2 = 1.0 / rs2;
     double s6 = s2 * s2 * s2;
-    a.pe += e4 * ((s6 * (s6 - 1.0)) + KA_C0 + KA_C2 * rs2);
-    double g = (2.0 * e4 * is2) * (6.0 * s6 * (s6 - 0.5) * s2 - KA_C2);
+    a.pe = fma(e4, fma(s6, s6, -s6) + fma(KA_C2, rs2, KA_C0), a.pe);
+    double g = (2.0 * e4 * is2) * fma(s6 * fma(6.0, s6, -3.0), s2, -KA_C2);
     double gl = g * L;
-    a.fx += gl * dx;
-    a.fy += gl * dy;
-    a.fz += gl * dz;
-    a.vir += g * dr2;
+    a.fx = fma(gl, dx, a.fx);
+    a.fy = fma(gl, dy, a.fy);
+    a.fz = fma(gl, dz, a.fz);
+    a.vir = fma(g, dr2, a.vir);
   }
 }
 
@@ -1030,8 +1034,8 @@ __device__ __forceinline__ void pair_fp32(PairAcc &a, const double4 &pi, int ti,
     const float e4 = tp == 0 ? 4.0f : (tp == 1 ? 6.0f : 2.0f);
     float s2 = __frcp_rn(rs2);
     float s6 = s2 * s2 * s2;
-    a.pe += (double)(e4 * ((s6 * (s6 - 1.0f)) + (float)KA_C0 + (float)KA_C2 * rs2));
-    float g = (2.0f * e4 * is2) * (6.0f * s6 * (s6 - 0.5f) * s2 - (float)KA_C2);
+    a.pe += (double)(e4 * (fmaf(s6, s6, -s6) + fmaf((float)KA_C2, rs2, (float)KA_C0)));
+    float g = (2.0f * e4 * is2) * fmaf(s6 * fmaf(6.0f, s6, -3.0f), s2, -(float)KA_C2);
     a.fx += (double)(g * dx);
     a.fy += (double)(g * dy);
     a.fz += (double)(g * dz);
@@ -2429,7 +2433,7 @@ __device__ __forceinline__ void particle_epilogue(const V &v, const SysDesc &d, 
     v.vx[i] = px;
     v.vy[i] = py;
     v.vz[i] = pz;
-    ke += px * px + py * py + pz * pz;
+    ke += fma(px, px, fma(py, py, __dmul_rn(pz, pz)));
   }
   pe += a.pe;
   vir += a.vir;
