@@ -172,6 +172,7 @@ struct SysState {
   double p_eps_end, p_eps_cur, eps_end, eps_cur;
   double u2[2];
   double brown_m[3];         // active Brownian (thermostat 6): mean random force of this step
+  int loaded, pad;           // the system holds a state (else it counts steps and nothing more)
 };
 
 // In-place observables of one system (set by acg_obs_configure): events of the

@@ -1027,7 +1027,7 @@ __device__ __forceinline__ void pair_fp32(PairAcc &a, const double4 &pi, int ti,
   const float Lf = (float)L;
   float dx = (float)min_image(pi.x - pj.x) * Lf, dy = (float)min_image(pi.y - pj.y) * Lf,
         dz = (float)min_image(pi.z - pj.z) * Lf;
-  float dr2 = dx * dx + dy * dy + dz * dz;
+  float dr2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
   const float is2 = tp == 0 ? 1.0f : (tp == 1 ? 1.5625f : (float)(1.0 / (0.88 * 0.88)));
   float rs2 = dr2 * is2;
   if (rs2 < (float)KA_RC2) {
@@ -1141,6 +1141,7 @@ __device__ void finalize_system(const View &v, int r, int mode, double4 *seg) {
 // (adjustInitialTemp, MDcode/initialise.c:141-151, with inst_T of
 // calculate_temp, :153-164), or none (NVE)
 __device__ __noinline__ void next_first_half(const SysDesc &d, SysState &st, SysDesc &dbox, double kb) {
+  if (!st.loaded) return;  // nothing to scale (and the box of a barostat waits too)
   if (st.ramp_left > 0) {
     const double inst = 2.0 * (kb * 0.5) / d.dof;
     st.s1 = sqrt(st.ramp_T / inst);
@@ -1221,6 +1222,16 @@ __device__ __noinline__ void finalize_sums(const SysDesc &d, SysState &st, SysDe
     st.ramp_left -= 1;
     st.ramp_real -= 1;
     if (st.ramp_left > 0) st.ramp_T = st.ramp_real > 0 ? __dadd_rn(st.ramp_T, st.ramp_dT) : st.ramp_end;
+  } else if (mode == 0 && !st.loaded) {
+    // no state yet: the step counter and the direction stream go on with the
+    // engine's other systems, the thermostat waits (on particles at rest its
+    // chain would run away, and the state loaded later would start from it)
+    st.step += 1;
+    if (st.shuf) {
+      st.mt_cur ^= 1;
+      st.shuf = 0;
+    }
+    return;
   } else if (mode == 0 && (d.thermostat == 2 || d.thermostat == 4)) {
     // advance_time_NVT_Berendsen (MDcode/time_evolve.c:173-256): after the
     // NVE step the momenta are scaled by chi = sqrt(1 + (T/inst_T - 1) dt /
@@ -1606,7 +1617,7 @@ __global__ void __launch_bounds__(BLOCK_A) k_brown_predict(View v) {
 // at the start of each step (not during a ramp) the box is rescaled and the
 // forces recomputed at the new length (force mode 3) before the kick.
 __device__ __forceinline__ bool npt_due(const SysDesc &d, const SysState &st) {
-  return d.thermostat == 4 && st.ramp_left == 0;
+  return d.thermostat == 4 && st.ramp_left == 0 && st.loaded;
 }
 
 // one thread per system: the pressure from the last forces' virial and
@@ -3461,6 +3472,7 @@ __global__ void __launch_bounds__(BLOCK_A) k_blank(View v) {
 
 __global__ void k_load(View v, int r) {
   const SysDesc &d = v.desc[r];
+  if (blockIdx.x == 0 && threadIdx.x == 0) v.st[r].loaded = 1;
   for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < d.n; k += gridDim.x * blockDim.x) {
     const int i = d.poff + k;
     const double *s = v.stage_d + 9 * (size_t)d.poff;

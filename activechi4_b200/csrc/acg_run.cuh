@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(NT, 1) k_run_box(View v, const int *order, int
       if (tid < nev && (ob.ev_info[ob_lo + tid] & 1) == 0) obs_accumulate(ob, n, ob.ev_info[ob_lo + tid], s_obs[tid]);
     }
     // ---- forces, second half kick, sums per 8 and per 32 slots
-    const bool nose = sd.thermostat == 1 && ramp == 0;
+    const bool nose = sd.thermostat == 1 && ramp == 0 && ss.loaded;
     if (nose && tid == NT - 32) s_half = nhc_before(ss.p_eta_cur, sd.rq, sd.T, sd.dt);
     for (int b = warp * (32 / TPP); b < 32 * nseg_own; b += NT / TPP) {
       const int k = b + lane / TPP;
