@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(BLOCK_A) k_observe(View v) {
 __global__ void k_flag_rebuild(View v, int all) {
   for (int s = threadIdx.x; s < v.nsys; s += blockDim.x) {
     SysState &st = v.st[s];
-    st.rebuild = all ? 1 : st.prime;
+    st.rebuild = all ? st.loaded : st.prime;
   }
 }
 
