@@ -34,10 +34,12 @@ namespace {
 constexpr int NA_BLOCK = 256;
 constexpr int NA_WARPS = NA_BLOCK / 32;
 constexpr int NA_MAX_BLOCKS = 8192;  // force blocks (each takes every NA_MAX_BLOCKS-th cell)
-// candidates of a cell's neighbourhood staged in shared memory: at density 1.2
-// a neighbourhood of 27 cells holds 750 to 1000 (up to 1250 where cells are
-// widest); with 40 bytes each four blocks of eight warps share an SM
+// candidates of a cell's neighbourhood staged in shared memory at a time: at
+// density 1.2 a neighbourhood of 27 cells holds 750 to 2000 (most where few
+// cells share a box not much under one cell more per side); with 40 bytes each
+// four blocks of eight warps share an SM
 constexpr int NA_CAP = 1280;
+constexpr int NA_FILL = 592;  // blocks that fill the 148 SMs
 constexpr size_t NA_SMEM = (size_t)NA_CAP * (sizeof(float4) + 3 * sizeof(double));
 
 // scratch layout (bytes): cell_of[N] order[N] ccount[C] cstart[C] cfill[C]
@@ -124,27 +126,86 @@ __global__ void k_na_scatter(NaArgs a) {
   na_i(a, OFF_ORDER)[slot] = i;
 }
 
+// the block's sums (pe, virial, active virial; one triple a warp, from lane 0)
+// stored as its partial sums; the last block to finish adds up all blocks' and
+// writes the scalars
+__device__ __forceinline__ void na_finish(const NaArgs &a, const double sum[3]) {
+  __shared__ double sh[3][NA_WARPS];
+  __shared__ int s_last;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (lane == 0)
+    for (int q = 0; q < 3; q++) sh[q][warp] = sum[q];
+  __syncthreads();
+  double *part = (double *)(a.scr + OFF_PART);
+  if (threadIdx.x == 0) {
+    for (int q = 0; q < 3; q++) {
+      double t = 0.0;
+      for (int ww = 0; ww < NA_WARPS; ww++) t += sh[q][ww];
+      part[4 * blockIdx.x + q] = t;
+    }
+    __threadfence();
+    s_last = atomicAdd((unsigned int *)(a.scr + OFF_CTR), 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  double t[3] = {0.0, 0.0, 0.0};
+  for (unsigned int b = threadIdx.x; b < gridDim.x; b += NA_BLOCK)
+    for (int q = 0; q < 3; q++) t[q] += __ldcg(&part[4 * b + q]);
+  for (int q = 0; q < 3; q++) {
+    for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_down_sync(0xffffffffu, t[q], o);
+    if (lane == 0) sh[q][warp] = t[q];
+  }
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  for (int q = 0; q < 3; q++) {
+    t[q] = 0.0;
+    for (int ww = 0; ww < NA_WARPS; ww++) t[q] += sh[q][ww];
+  }
+  a.out[0] = 0.5 * t[0];
+  a.out[1] = (0.5 * t[1]) / 3.0;
+  a.out[2] = t[2];
+  *(unsigned int *)(a.scr + OFF_CTR) = 0u;
+}
+
+// the active force of particle i (MDcode/cell_list+forces.c:207-218) added to
+// its pair force; returns its active virial
+__device__ __forceinline__ double na_active(const NaArgs &a, int i, acg::PairAcc &acc) {
+  const int t = a.act[i];
+  if (t < 0 || t >= a.nact) return 0.0;
+  const double kx = (double)a.k[t], ky = (double)a.k[a.nact + t], kz = (double)a.k[2 * a.nact + t];
+  const double *u = a.xu ? a.xu : a.x;
+  acc.fx += a.f0 * kx;
+  acc.fy += a.f0 * ky;
+  acc.fz += a.f0 * kz;
+  return a.f0 * (kx * u[3 * i] + ky * u[3 * i + 1] + kz * u[3 * i + 2]);
+}
+
 // Forces by cells: one block stages a cell's 27 neighbour cells (8 at two cells
-// per side) once -- FP32 reduced coordinates with index and type for the
-// distance test, FP64 ones for the pair terms -- and its warps take the cell's
-// particles one at a time: the lanes test 32 candidates a step in FP32 against
-// the pair's own cut widened by 1e-4 (the coordinates' rounding is below 2e-5 of
-// it at the largest box), the accepted ones queue up, and every 32 of them are
-// evaluated by a full warp in FP64 (masked by the exact cut).  About one
-// candidate in twelve is within the cut, so the FP64 terms, which bounded a
-// version that evaluated each candidate under a branch, run on full warps.
-// What bounds it now: issue (about 50 instructions per 32 candidates tested).
-// N = 20000: 260 -> 100 us a call with the cell build.
-// A neighbourhood above NA_CAP candidates is evaluated straight from memory.
-__global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
+// per side) -- FP32 reduced coordinates with index and type for the distance
+// test, FP64 ones for the pair terms -- and its warps take the cell's particles
+// one at a time: the lanes test 32 candidates a step in FP32 against the pair's
+// own cut widened by 1e-4 (the coordinates' rounding is below 2e-5 of it at the
+// largest box), the accepted ones queue up, and every 32 of them are evaluated by
+// a full warp in FP64 (masked by the exact cut).  About one candidate in twelve is
+// within the cut, so the FP64 terms, which bounded a version that evaluated
+// each candidate under a branch, run on full warps.  What bounds it now: issue
+// (about 50 instructions per 32 candidates tested).  N = 20000: 260 -> 101 us a
+// call with the cell build.
+//
+// A neighbourhood of more than NA_CAP candidates is taken in pieces of that many,
+// each particle's force carried from one piece to the next in F (evaluated straight
+// from memory such a cell made a call of N = 2000 take 597 us against 155 for the
+// version of four threads a particle; in pieces 54).  A cell of a grid of few
+// cells is shared by `split` blocks that stage the same neighbourhood: N = 700 78
+// -> 30 us, N = 5000 76 -> 56.
+__global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a, int split) {
   extern __shared__ __align__(16) unsigned char na_sm[];
   float4 *cf = reinterpret_cast<float4 *>(na_sm);
   double *cx = reinterpret_cast<double *>(na_sm + NA_CAP * sizeof(float4)), *cy = cx + NA_CAP, *cz = cy + NA_CAP;
   __shared__ int s_pre[28], s_start[27];
   __shared__ uint16_t queue[NA_WARPS][96];
   __shared__ signed char s_img[3][27];  // image of each neighbour cell (3 and more cells per side)
-  __shared__ double sh[3][NA_WARPS];
-  __shared__ int s_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int nc = a.nc, ncell = nc * nc * nc;
   const int lo = acg::stencil_lo(nc), wd = acg::stencil_hi(nc) - lo + 1, ns = wd * wd * wd;
@@ -154,7 +215,8 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
   float cut[3];  // the test's cuts by type sum, reduced units
   for (int k = 0; k < 3; k++) cut[k] = (float)(acg::KA_RC2 * (1.0 + 1e-4) / (acg::ka_is2(k) * L * L));
   double sum[3] = {0.0, 0.0, 0.0};  // pe, virial, active virial of this warp's particles (lane 0)
-  for (int c = blockIdx.x; c < ncell; c += gridDim.x) {
+  for (int b = blockIdx.x; b < ncell * split; b += gridDim.x) {
+    const int c = b / split, part = b - c * split;
     if (warp == 0) {
       int m = 0;
       if (lane < ns) {
@@ -177,12 +239,12 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
       if (lane == 0) s_pre[0] = 0;
     }
     __syncthreads();
-    const int Q = s_pre[ns], mc = s_pre[own + 1] - s_pre[own];
-    const bool staged = Q <= NA_CAP;
-    if (staged && mc > 0)
-      for (int q = threadIdx.x; q < Q; q += NA_BLOCK) {
-        const int u = acg::union_of(s_pre, ns, q);
-        const int j = order[s_start[u] + (q - s_pre[u])];
+    const int mc = s_pre[own + 1] - s_pre[own], Q = part * NA_WARPS < mc ? s_pre[ns] : 0;
+    for (int p0 = 0; p0 < Q; p0 += NA_CAP) {
+      const int np = min(Q - p0, NA_CAP);
+      for (int q = threadIdx.x; q < np; q += NA_BLOCK) {
+        const int u = acg::union_of(s_pre, ns, p0 + q);
+        const int j = order[s_start[u] + (p0 + q - s_pre[u])];
         const double x = a.x[3 * j], y = a.x[3 * j + 1], z = a.x[3 * j + 2];
         cf[q] = make_float4((float)(x + s_img[0][u]), (float)(y + s_img[1][u]), (float)(z + s_img[2][u]),
                             __int_as_float(j | (a.type[j] << 30)));
@@ -190,16 +252,17 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
         cy[q] = y;
         cz[q] = z;
       }
-    __syncthreads();
-    for (int w = warp; w < mc; w += NA_WARPS) {
-      const int i = order[s_start[own] + w];
-      const int ti = a.type[i];
-      const acg::PairParamsD P(ti, L);
-      acg::PairAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
-      if (staged) {
-        const int qi = s_pre[own] + w;
-        const float4 fi = cf[qi];
-        const double xi = cx[qi], yi = cy[qi], zi = cz[qi];
+      __syncthreads();
+      for (int w = part * NA_WARPS + warp; w < mc; w += NA_WARPS * split) {
+        const int i = order[s_start[own] + w];
+        const int ti = a.type[i];
+        const acg::PairParamsD P(ti, L);
+        acg::PairAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+        const int qi = s_pre[own] + w - p0;  // the particle itself among the piece's
+        const bool here = qi >= 0 && qi < np;
+        const double xi = here ? cx[qi] : a.x[3 * i], yi = here ? cy[qi] : a.x[3 * i + 1],
+                     zi = here ? cz[qi] : a.x[3 * i + 2];
+        const float fx = (float)xi, fy = (float)yi, fz = (float)zi;
         const float c0 = ti == 0 ? cut[0] : cut[1], c1 = ti == 0 ? cut[1] : cut[2];
         uint16_t *qu = queue[warp];
         int cnt = 0;
@@ -212,9 +275,9 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
           __syncwarp();
         };
         auto test = [&](int q) {
-          if (q >= Q) return false;
+          if (q >= np) return false;
           const float4 fj = cf[q];
-          float dx = fi.x - fj.x, dy = fi.y - fj.y, dz = fi.z - fj.z;
+          float dx = fx - fj.x, dy = fy - fj.y, dz = fz - fj.z;
           if (nc < 3) {  // every cell neighbours every other under two images
             dx -= rintf(dx);
             dy -= rintf(dy);
@@ -223,7 +286,7 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
           return fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < (((__float_as_int(fj.w) >> 30) & 1) ? c1 : c0) && q != qi;
         };
         const unsigned below = (1u << lane) - 1u;
-        for (int q0 = lane; q0 - lane < Q; q0 += 64) {
+        for (int q0 = lane; q0 - lane < np; q0 += 64) {
           const bool ok0 = test(q0), ok1 = test(q0 + 32);
           const unsigned b0 = __ballot_sync(0xffffffffu, ok0), b1 = __ballot_sync(0xffffffffu, ok1);
           if (ok0) qu[cnt + __popc(b0 & below)] = (uint16_t)q0;
@@ -233,78 +296,35 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a) {
           while (cnt >= 32) pairs(32);
         }
         if (cnt > 0) pairs(cnt);
-      } else {
-        const double xi = a.x[3 * i], yi = a.x[3 * i + 1], zi = a.x[3 * i + 2];
-        for (int u = 0; u < ns; u++)
-          for (int q = lane; q < s_pre[u + 1] - s_pre[u]; q += 32) {
-            const int j = order[s_start[u] + q];
-            if (j != i)
-              acg::pair_f64(acc, acg::min_image(xi - a.x[3 * j]), acg::min_image(yi - a.x[3 * j + 1]),
-                            acg::min_image(zi - a.x[3 * j + 2]), P, a.type[j] != 0, true);
-          }
-      }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        acc.fx += __shfl_xor_sync(0xffffffffu, acc.fx, o);
-        acc.fy += __shfl_xor_sync(0xffffffffu, acc.fy, o);
-        acc.fz += __shfl_xor_sync(0xffffffffu, acc.fz, o);
-        acc.pe += __shfl_xor_sync(0xffffffffu, acc.pe, o);
-        acc.vir += __shfl_xor_sync(0xffffffffu, acc.vir, o);
-      }
-      if (lane == 0) {
-        acg::pair_scale(acc, L);
-        const int t = a.act[i];
-        if (t >= 0 && t < a.nact) {  // active force (MDcode/cell_list+forces.c:207-218)
-          const double kx = (double)a.k[t], ky = (double)a.k[a.nact + t], kz = (double)a.k[2 * a.nact + t];
-          const double *u = a.xu ? a.xu : a.x;
-          acc.fx += a.f0 * kx;
-          acc.fy += a.f0 * ky;
-          acc.fz += a.f0 * kz;
-          sum[2] += a.f0 * (kx * u[3 * i] + ky * u[3 * i + 1] + kz * u[3 * i + 2]);
+        for (int o = 16; o > 0; o >>= 1) {
+          acc.fx += __shfl_xor_sync(0xffffffffu, acc.fx, o);
+          acc.fy += __shfl_xor_sync(0xffffffffu, acc.fy, o);
+          acc.fz += __shfl_xor_sync(0xffffffffu, acc.fz, o);
+          acc.pe += __shfl_xor_sync(0xffffffffu, acc.pe, o);
+          acc.vir += __shfl_xor_sync(0xffffffffu, acc.vir, o);
         }
-        a.F[3 * i] = acc.fx;
-        a.F[3 * i + 1] = acc.fy;
-        a.F[3 * i + 2] = acc.fz;
-        sum[0] += acc.pe;
-        sum[1] += acc.vir;
+        if (lane == 0) {
+          acg::pair_scale(acc, L);
+          if (p0 == 0) {
+            sum[2] += na_active(a, i, acc);
+          } else {
+            acc.fx += a.F[3 * i];
+            acc.fy += a.F[3 * i + 1];
+            acc.fz += a.F[3 * i + 2];
+          }
+          a.F[3 * i] = acc.fx;
+          a.F[3 * i + 1] = acc.fy;
+          a.F[3 * i + 2] = acc.fz;
+          sum[0] += acc.pe;
+          sum[1] += acc.vir;
+        }
       }
+      __syncthreads();
     }
     __syncthreads();
   }
-  if (lane == 0)
-    for (int q = 0; q < 3; q++) sh[q][warp] = sum[q];
-  __syncthreads();
-  double *part = (double *)(a.scr + OFF_PART);
-  if (threadIdx.x == 0) {
-    for (int q = 0; q < 3; q++) {
-      double t = 0.0;
-      for (int ww = 0; ww < NA_WARPS; ww++) t += sh[q][ww];
-      part[4 * blockIdx.x + q] = t;
-    }
-    __threadfence();
-    s_last = atomicAdd((unsigned int *)(a.scr + OFF_CTR), 1u) == gridDim.x - 1;
-  }
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  // the last block adds up all blocks' sums
-  double t[3] = {0.0, 0.0, 0.0};
-  for (unsigned int b = threadIdx.x; b < gridDim.x; b += NA_BLOCK)
-    for (int q = 0; q < 3; q++) t[q] += __ldcg(&part[4 * b + q]);
-  for (int q = 0; q < 3; q++) {
-    for (int o = 16; o > 0; o >>= 1) t[q] += __shfl_down_sync(0xffffffffu, t[q], o);
-    if (lane == 0) sh[q][warp] = t[q];
-  }
-  __syncthreads();
-  if (threadIdx.x != 0) return;
-  for (int q = 0; q < 3; q++) {
-    t[q] = 0.0;
-    for (int ww = 0; ww < NA_WARPS; ww++) t[q] += sh[q][ww];
-  }
-  a.out[0] = 0.5 * t[0];
-  a.out[1] = (0.5 * t[1]) / 3.0;
-  a.out[2] = t[2];
-  *(unsigned int *)(a.scr + OFF_CTR) = 0u;
+  na_finish(a, sum);
 }
 
 }  // namespace
@@ -371,7 +391,10 @@ extern "C" int acg_forces_noalloc(const double *x, const double *xu, const int *
   k_na_count<<<(n + 255) / 256, 256, 0, s>>>(a);
   k_na_scan<<<1, 1024, 0, s>>>(a);
   k_na_scatter<<<(n + 255) / 256, 256, 0, s>>>(a);
-  k_na_force<<<std::min(ncell, NA_MAX_BLOCKS), NA_BLOCK, NA_SMEM, s>>>(a);
+  // blocks sharing a cell: as many as fill the chip, with a particle for each
+  // warp on average
+  const int split = std::max(1, std::min(NA_FILL / ncell, (n + NA_WARPS * ncell - 1) / (NA_WARPS * ncell)));
+  k_na_force<<<std::min(ncell * split, NA_MAX_BLOCKS), NA_BLOCK, NA_SMEM, s>>>(a, split);
   ce = cudaGetLastError();
   if (ce != cudaSuccess)
     return na_fail(ACG_ERR_CUDA, std::string("acg_forces_noalloc: launch: ") + cudaGetErrorString(ce));
