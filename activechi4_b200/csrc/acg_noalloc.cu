@@ -199,6 +199,8 @@ __device__ __forceinline__ double na_active(const NaArgs &a, int i, acg::PairAcc
 // version of four threads a particle; in pieces 54).  A cell of a grid of few
 // cells is shared by `split` blocks that stage the same neighbourhood: N = 700 78
 // -> 30 us, N = 5000 76 -> 56.
+// Coordinates outside [0, 1] get the minimum image in the test (the cells' images
+// say nothing about them).
 __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a, int split) {
   extern __shared__ __align__(16) unsigned char na_sm[];
   float4 *cf = reinterpret_cast<float4 *>(na_sm);
@@ -214,6 +216,9 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a, int split) {
   const int *order = na_i(a, OFF_ORDER);
   float cut[3];  // the test's cuts by type sum, reduced units
   for (int k = 0; k < 3; k++) cut[k] = (float)(acg::KA_RC2 * (1.0 + 1e-4) / (acg::ka_is2(k) * L * L));
+  auto outside = [](double x, double y, double z) {
+    return !(x >= 0.0 && x <= 1.0 && y >= 0.0 && y <= 1.0 && z >= 0.0 && z <= 1.0);
+  };
   double sum[3] = {0.0, 0.0, 0.0};  // pe, virial, active virial of this warp's particles (lane 0)
   for (int b = blockIdx.x; b < ncell * split; b += gridDim.x) {
     const int c = b / split, part = b - c * split;
@@ -242,17 +247,25 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a, int split) {
     const int mc = s_pre[own + 1] - s_pre[own], Q = part * NA_WARPS < mc ? s_pre[ns] : 0;
     for (int p0 = 0; p0 < Q; p0 += NA_CAP) {
       const int np = min(Q - p0, NA_CAP);
+      bool out = false;
       for (int q = threadIdx.x; q < np; q += NA_BLOCK) {
         const int u = acg::union_of(s_pre, ns, p0 + q);
         const int j = order[s_start[u] + (p0 + q - s_pre[u])];
         const double x = a.x[3 * j], y = a.x[3 * j + 1], z = a.x[3 * j + 2];
+        out |= outside(x, y, z);
         cf[q] = make_float4((float)(x + s_img[0][u]), (float)(y + s_img[1][u]), (float)(z + s_img[2][u]),
                             __int_as_float(j | (a.type[j] << 30)));
         cx[q] = x;
         cy[q] = y;
         cz[q] = z;
       }
-      __syncthreads();
+      const bool far = __syncthreads_or(out);
+      if (far) {
+        for (int q = threadIdx.x; q < np; q += NA_BLOCK)
+          cf[q] = make_float4((float)acg::min_image(cx[q]), (float)acg::min_image(cy[q]),
+                              (float)acg::min_image(cz[q]), cf[q].w);
+        __syncthreads();
+      }
       for (int w = part * NA_WARPS + warp; w < mc; w += NA_WARPS * split) {
         const int i = order[s_start[own] + w];
         const int ti = a.type[i];
@@ -262,7 +275,11 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a, int split) {
         const bool here = qi >= 0 && qi < np;
         const double xi = here ? cx[qi] : a.x[3 * i], yi = here ? cy[qi] : a.x[3 * i + 1],
                      zi = here ? cz[qi] : a.x[3 * i + 2];
-        const float fx = (float)xi, fy = (float)yi, fz = (float)zi;
+        const bool fold = far || outside(xi, yi, zi);
+        // (at two cells per side every cell neighbours every other under two images)
+        const bool image = fold || nc < 3;
+        const float fx = (float)(fold ? acg::min_image(xi) : xi), fy = (float)(fold ? acg::min_image(yi) : yi),
+                    fz = (float)(fold ? acg::min_image(zi) : zi);
         const float c0 = ti == 0 ? cut[0] : cut[1], c1 = ti == 0 ? cut[1] : cut[2];
         uint16_t *qu = queue[warp];
         int cnt = 0;
@@ -278,7 +295,7 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a, int split) {
           if (q >= np) return false;
           const float4 fj = cf[q];
           float dx = fx - fj.x, dy = fy - fj.y, dz = fz - fj.z;
-          if (nc < 3) {  // every cell neighbours every other under two images
+          if (image) {
             dx -= rintf(dx);
             dy -= rintf(dy);
             dz -= rintf(dz);

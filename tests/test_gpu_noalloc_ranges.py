@@ -1,7 +1,8 @@
 """The allocation-free forces where their split of the work changes: pieces of a
 neighbourhood above the staged capacity with the cell itself in the first, a
 later or two pieces, cells shared by several blocks, the most cells (32 per side, where the FP32 test's margin is tightest, with pairs on both
-sides of each cut and across the faces), droplets in an empty box; particles whose position is no number.  Forces, energy, virial
+sides of each cut and across the faces), droplets in an empty box; coordinates
+outside [0, 1); particles whose position is no number.  Forces, energy, virial
 and active virial against a plain FP64 sum in torch; tolerance: the entry point's
 documented 1e-12 of the rms force (the scalars: of the sum of the magnitudes of
 the terms that a pair's energy and virial are made of; at the cut these cancel)."""
@@ -141,6 +142,20 @@ def test_droplet(cuda_lib):
     l = (n / 1.3) ** (1.0 / 3.0)
     x = (_grid(n, l, rng) - 0.5) * l / L
     _check(cuda_lib, x % 1.0, (rng.random(n) < 0.2).astype(np.int32), L, 5)
+
+
+@pytest.mark.parametrize("n", [700, 1000, 1500])
+@pytest.mark.parametrize("most", [1, 5, 100000])
+def test_unfolded(cuda_lib, n, most):
+    """Up to three cells per side every cell neighbours every other, so the sums
+    never depended on the coordinates being folded into the box."""
+    rng = np.random.default_rng(n + most)
+    L = (n / 1.2) ** (1.0 / 3.0)
+    # whole boxes away: the folded coordinates are exact multiples of 2^-32
+    x = np.floor(_grid(n, L, rng) * 2.0 ** 32) / 2.0 ** 32
+    some = rng.random(n) < 0.3
+    x[some] += rng.integers(-most, most + 1, (some.sum(), 3))
+    _check(cuda_lib, x, (rng.random(n) < 0.2).astype(np.int32), L, 11)
 
 
 @pytest.mark.parametrize("n,density", [(700, 1.2), (1500, 1.2), (1500, 6.0), (3500, 1.2)])
