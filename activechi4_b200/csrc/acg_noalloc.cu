@@ -40,6 +40,13 @@ constexpr int NA_MAX_BLOCKS = 8192;  // force blocks (each takes every NA_MAX_BL
 // four blocks of eight warps share an SM
 constexpr int NA_CAP = 1280;
 constexpr int NA_FILL = 592;  // blocks that fill the 148 SMs
+// below this many particles a cell, on grids of at least this many cells, the
+// forces go particle by particle (us a call, by cells / by particles: 14 to 17
+// cells per side 89 / 49 at one particle a cell, 57 / 50 at 2.4, 80 / 68 at 4.1,
+// 74 / 74 at 4.9; 12 per side, all of whose cells fit on the chip in three waves,
+// 37 / 41 at 1.2; the larger grids lie between: 27 per side 161 / 59 at one, 234 /
+// 235 at 5.1)
+constexpr int NA_SPARSE = 4, NA_SPARSE_CELLS = 14 * 14 * 14;
 constexpr size_t NA_SMEM = (size_t)NA_CAP * (sizeof(float4) + 3 * sizeof(double));
 
 // scratch layout (bytes): cell_of[N] order[N] ccount[C] cstart[C] cfill[C]
@@ -344,6 +351,60 @@ __global__ void __launch_bounds__(NA_BLOCK, 4) k_na_force(NaArgs a, int split) {
   na_finish(a, sum);
 }
 
+// Forces by particles, for large grids of few particles a cell: four threads take a particle's neighbour cells one after another,
+// straight from memory.  Staging a neighbourhood of a few dozen candidates costs
+// k_na_force a block and its barriers for a particle or two.
+constexpr int NA_TPP = 4;
+__global__ void __launch_bounds__(NA_BLOCK) k_na_force_sparse(NaArgs a) {
+  const int i = (blockIdx.x * NA_BLOCK + threadIdx.x) / NA_TPP, lane = threadIdx.x % NA_TPP;
+  const double L = a.L;
+  acg::PairAcc acc = {0.0, 0.0, 0.0, 0.0, 0.0};
+  double va = 0.0;
+  if (i < a.n) {
+    const double xi = a.x[3 * i], yi = a.x[3 * i + 1], zi = a.x[3 * i + 2];
+    const acg::PairParamsD P(a.type[i], L);
+    const int nc = a.nc, c = na_i(a, OFF_CELL)[i];
+    const int cx = c % nc, cy = (c / nc) % nc, cz = c / (nc * nc);
+    const int lo = acg::stencil_lo(nc), hi = acg::stencil_hi(nc);
+    for (int oz = lo; oz <= hi; oz++)
+      for (int oy = lo; oy <= hi; oy++)
+        for (int ox = lo; ox <= hi; ox++) {
+          const int c2 = acg::wrap_cell(cx + ox, nc) + acg::wrap_cell(cy + oy, nc) * nc +
+                         acg::wrap_cell(cz + oz, nc) * nc * nc;
+          const int s0 = na_i(a, OFF_START)[c2], m = na_i(a, OFF_COUNT)[c2];
+          for (int q = lane; q < m; q += NA_TPP) {
+            const int j = na_i(a, OFF_ORDER)[s0 + q];
+            if (j == i) continue;
+            const double dx = acg::min_image(xi - a.x[3 * j]), dy = acg::min_image(yi - a.x[3 * j + 1]),
+                         dz = acg::min_image(zi - a.x[3 * j + 2]);
+            const bool tj = a.type[j] != 0;
+            if (fma(dx, dx, fma(dy, dy, dz * dz)) * P.is2[tj] < acg::KA_RC2)
+              acg::pair_f64(acc, dx, dy, dz, P, tj, true);
+          }
+        }
+  }
+#pragma unroll
+  for (int o = NA_TPP / 2; o > 0; o >>= 1) {
+    acc.fx += __shfl_xor_sync(0xffffffffu, acc.fx, o);
+    acc.fy += __shfl_xor_sync(0xffffffffu, acc.fy, o);
+    acc.fz += __shfl_xor_sync(0xffffffffu, acc.fz, o);
+    acc.pe += __shfl_xor_sync(0xffffffffu, acc.pe, o);
+    acc.vir += __shfl_xor_sync(0xffffffffu, acc.vir, o);
+  }
+  const bool mine = i < a.n && lane == 0;
+  if (mine) {
+    acg::pair_scale(acc, L);
+    va = na_active(a, i, acc);
+    a.F[3 * i] = acc.fx;
+    a.F[3 * i + 1] = acc.fy;
+    a.F[3 * i + 2] = acc.fz;
+  }
+  double sum[3] = {mine ? acc.pe : 0.0, mine ? acc.vir : 0.0, va};
+  for (int q = 0; q < 3; q++)
+    for (int o = 16; o > 0; o >>= 1) sum[q] += __shfl_down_sync(0xffffffffu, sum[q], o);
+  na_finish(a, sum);
+}
+
 }  // namespace
 
 extern "C" int acg_forces_noalloc(const double *x, const double *xu, const int *type, const int *act_tag,
@@ -408,10 +469,14 @@ extern "C" int acg_forces_noalloc(const double *x, const double *xu, const int *
   k_na_count<<<(n + 255) / 256, 256, 0, s>>>(a);
   k_na_scan<<<1, 1024, 0, s>>>(a);
   k_na_scatter<<<(n + 255) / 256, 256, 0, s>>>(a);
-  // blocks sharing a cell: as many as fill the chip, with a particle for each
-  // warp on average
-  const int split = std::max(1, std::min(NA_FILL / ncell, (n + NA_WARPS * ncell - 1) / (NA_WARPS * ncell)));
-  k_na_force<<<std::min(ncell * split, NA_MAX_BLOCKS), NA_BLOCK, NA_SMEM, s>>>(a, split);
+  if (ncell >= NA_SPARSE_CELLS && n < NA_SPARSE * ncell) {
+    k_na_force_sparse<<<(n * NA_TPP + NA_BLOCK - 1) / NA_BLOCK, NA_BLOCK, 0, s>>>(a);
+  } else {
+    // blocks sharing a cell: as many as fill the chip, with a particle for each
+    // warp on average
+    const int split = std::max(1, std::min(NA_FILL / ncell, (n + NA_WARPS * ncell - 1) / (NA_WARPS * ncell)));
+    k_na_force<<<std::min(ncell * split, NA_MAX_BLOCKS), NA_BLOCK, NA_SMEM, s>>>(a, split);
+  }
   ce = cudaGetLastError();
   if (ce != cudaSuccess)
     return na_fail(ACG_ERR_CUDA, std::string("acg_forces_noalloc: launch: ") + cudaGetErrorString(ce));

@@ -1,6 +1,8 @@
 """The allocation-free forces where their split of the work changes: pieces of a
 neighbourhood above the staged capacity with the cell itself in the first, a
-later or two pieces, cells shared by several blocks, the most cells (32 per side, where the FP32 test's margin is tightest, with pairs on both
+later or two pieces, cells shared by several blocks, grids of few particles a
+cell (by particles from 14 cells per side on, fewer than four a cell), the most
+cells (32 per side, where the FP32 test's margin is tightest, with pairs on both
 sides of each cut and across the faces), droplets in an empty box; coordinates
 outside [0, 1); particles whose position is no number.  Forces, energy, virial
 and active virial against a plain FP64 sum in torch; tolerance: the entry point's
@@ -92,7 +94,8 @@ def _grid(n, L, rng, jitter=0.05):
 
 @pytest.mark.parametrize("n,density", [
     (1280, 1.2), (1281, 1.2), (1500, 1.2), (2561, 2.2), (3000, 6.0), (3041, 1.2), (6500, 1.2),  # pieces
-    (277, 1.2), (700, 1.2), (1000, 1.2), (4100, 1.2), (9000, 1.2), (15000, 2.5)])                 # shared cells
+    (277, 1.2), (700, 1.2), (1000, 1.2), (4100, 1.2), (9000, 1.2), (15000, 2.5),                  # shared cells
+    (10975, 0.175), (10976, 0.175), (10977, 0.175), (8788, 0.175), (3000, 0.03), (64, 0.004)])    # few a cell
 def test_split(cuda_lib, n, density):
     rng = np.random.default_rng(n)
     L = (n / density) ** (1.0 / 3.0)
@@ -120,7 +123,7 @@ def _pairs_at_cuts(L, rng):
 
 @pytest.mark.parametrize("fill", [0, 140000])
 def test_most_cells(cuda_lib, fill):
-    """32 cells per side; without and with other particles."""
+    """32 cells per side; without and with other particles (by particles, by cells)."""
     rng = np.random.default_rng(fill)
     L = 93.9
     x, typ = _pairs_at_cuts(L, rng)
@@ -158,7 +161,7 @@ def test_unfolded(cuda_lib, n, most):
     _check(cuda_lib, x, (rng.random(n) < 0.2).astype(np.int32), L, 11)
 
 
-@pytest.mark.parametrize("n,density", [(700, 1.2), (1500, 1.2), (1500, 6.0), (3500, 1.2)])
+@pytest.mark.parametrize("n,density", [(700, 1.2), (1500, 1.2), (1500, 6.0), (3500, 1.2), (8000, 0.02)])
 @pytest.mark.parametrize("bad", [np.nan, np.inf])
 def test_no_number(cuda_lib, n, density, bad):
     """A particle whose position is no number takes part in no pair."""
