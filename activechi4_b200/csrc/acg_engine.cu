@@ -248,9 +248,9 @@ struct acg_engine {
   int tpp = 4, block = 128, gtpp = 2, btpp = 2;  // btpp: whole-box kernels
   int ntiles_a = 0, ntiles_b = 0, ntiles_l = 0, ntiles_c = 0, ntiles_g = 0, ntiles_x = 0, ntiles_lc = 0;
   // whole runs in one launch (k_run_box): blocks per cluster (0: the engine
-  // steps kernel by kernel), threads per block, state in shared memory, dynamic
-  // shared memory, systems in launch order (device)
-  int run_c = 0, run_nt = 0, run_resident = 0;
+  // steps kernel by kernel), state in shared memory, dynamic shared memory,
+  // systems in launch order (device)
+  int run_c = 0, run_resident = 0;
   size_t run_smem = 0;
   int *run_order = nullptr;
   int2 *d_tiles_b = nullptr;
@@ -350,10 +350,13 @@ RunFn run_fn_of(int tpp) {
   }
   return nullptr;
 }
-RunFn run_fn(int tpp, int prec, int nt, bool resident) {
+// threads per block: 512 where FP64 pair terms take about 120 registers a
+// thread, or where the state fits in shared memory (few slots a block); 1024 for
+// FP32 with the state in L2 (never up to 256 slots a block, where everything fits)
+int run_threads(int prec, bool resident) { return prec && !resident ? 1024 : 512; }
+RunFn run_fn(int tpp, int prec, bool resident) {
   if (!prec) return resident ? run_fn_of<0, 512, true>(tpp) : run_fn_of<0, 512, false>(tpp);
-  if (resident) return run_fn_of<1, 512, true>(tpp);
-  return nt == 512 ? run_fn_of<1, 512, false>(tpp) : run_fn_of<1, 1024, false>(tpp);
+  return resident ? run_fn_of<1, 512, true>(tpp) : run_fn_of<1, 1024, false>(tpp);
 }
 
 // whether one system can run inside a cluster: whole-box lists from sub-cells,
@@ -376,13 +379,9 @@ void plan_run(acg_engine *e, size_t smem_limit) {
     if (!run_eligible(L.desc[r])) return;
   const int C0 = L.nsys <= 7 ? 16 : (L.nsys <= 15 ? 8 : (L.nsys <= 33 ? 4 : (L.nsys <= 74 ? 2 : 1)));
   const int prec = L.desc[0].precision;
-  // state in shared memory where it fits; threads per block: 512 (FP64 pair
-  // terms take about 120 registers a thread), or 1024 for FP32 systems with
-  // more slots per block than that
+  // state in shared memory where it fits
   for (int C = C0, resident = 1; C <= 16; C = resident ? C : 2 * C, resident ^= 1) {
-    int nloc = 0;
-    for (const SysDesc &d : L.desc) nloc = std::max(nloc, 32 * (((d.n + 31) / 32 + C - 1) / C));
-    const int nt = prec && !resident && nloc * 2 > 512 ? 1024 : 512;
+    const int nt = run_threads(prec, resident);
     size_t least = 0, want = 0;
     for (const SysDesc &d : L.desc) {
       const RunPlan p = run_plan(d.n, d.ncell, d.msub, prec, C, resident, nt / 32);
@@ -394,7 +393,6 @@ void plan_run(acg_engine *e, size_t smem_limit) {
     }
     if (least > smem_limit) continue;
     e->run_c = C;
-    e->run_nt = nt;
     e->run_resident = resident;
     e->run_smem = std::min(smem_limit, std::max(least, want));
     return;
@@ -404,7 +402,7 @@ void plan_run(acg_engine *e, size_t smem_limit) {
 void run_config(const acg_engine *e, cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at) {
   cfg = {};
   cfg.gridDim = dim3(e->lay.nsys * e->run_c);
-  cfg.blockDim = dim3(e->run_nt);
+  cfg.blockDim = dim3(run_threads(e->lay.desc[0].precision, e->run_resident));
   cfg.dynamicSmemBytes = e->run_smem;
   cfg.stream = e->stream;
   at.id = cudaLaunchAttributeClusterDimension;
@@ -419,7 +417,7 @@ int launch_run(acg_engine *e, int nsteps) {
   cudaLaunchConfig_t cfg;
   cudaLaunchAttribute at;
   run_config(e, cfg, at);
-  CK(cudaLaunchKernelEx(&cfg, run_fn(e->btpp, e->lay.desc[0].precision, e->run_nt, e->run_resident), e->v,
+  CK(cudaLaunchKernelEx(&cfg, run_fn(e->btpp, e->lay.desc[0].precision, e->run_resident), e->v,
                         (const int *)e->run_order, nsteps, (unsigned)e->run_smem));
   return ACG_OK;
 }
@@ -1210,7 +1208,7 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
     std::stable_sort(ord.begin(), ord.end(), [&](int a, int b) { return L.desc[a].n > L.desc[b].n; });
     run_order.swap(ord);
     for (int gt : {1, 2, 4}) {
-      const void *fn = (const void *)run_fn(gt, L.desc[0].precision, e->run_nt, e->run_resident);
+      const void *fn = (const void *)run_fn(gt, L.desc[0].precision, e->run_resident);
       bool ok = raise_smem(fn, e->run_smem);
       if (ok && e->run_c > 8)
         ok = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
@@ -1948,6 +1946,17 @@ int acg_get_launch(acg_engine *e, int *tpp, int *block) {
   if (!e) return fail(ACG_ERR_INVALID, "null engine");
   if (tpp) *tpp = e->tpp;
   if (block) *block = e->block;
+  return ACG_OK;
+}
+
+int acg_get_run_plan(acg_engine *e, int *cluster, int *threads, int *resident, int *min_steps, int *max_steps) {
+  if (!e) return fail(ACG_ERR_INVALID, "null engine");
+  const bool run = e->run_c > 0;
+  if (cluster) *cluster = e->run_c;
+  if (threads) *threads = run ? run_threads(e->lay.desc[0].precision, e->run_resident) : 0;
+  if (resident) *resident = run && e->run_resident;
+  if (min_steps) *min_steps = run ? 1 : 0;
+  if (max_steps) *max_steps = run ? RUN_STEPS : 0;
   return ACG_OK;
 }
 

@@ -314,6 +314,14 @@ class Engine:
         check(self._lib.acg_get_box_cells(self.h, C.byref(c)))
         return c.value
 
+    def run_plan(self) -> dict:
+        """How `step` advances the engine: blocks of each system's cluster (0:
+        kernel by kernel), threads per block, state in shared memory, fewest
+        steps of a call and most steps of a launch that run this way."""
+        v = [C.c_int() for _ in range(5)]
+        check(self._lib.acg_get_run_plan(self.h, *(C.byref(x) for x in v)))
+        return dict(zip(("cluster", "threads", "resident", "min_steps", "max_steps"), (x.value for x in v)))
+
     def get_launch(self):
         t, b = C.c_int(), C.c_int()
         check(self._lib.acg_get_launch(self.h, C.byref(t), C.byref(b)))

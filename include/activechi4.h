@@ -239,9 +239,12 @@ int acg_compute_forces(acg_engine *e);
  * when due (MDcode/main.c:245-247) then AdvanceTimeNVTNoseHoover
  * (MDcode/time_evolve.c:495-526) or advance_time_NVEFrog
  * (MDcode/time_evolve.c:104-171).  Runs as CUDA-graph launches on the
- * engine's stream, or, where every system has 2 to 4 cells per side, as one
- * kernel that advances each system inside a thread-block cluster; returns after
- * queuing (acg_sync waits). */
+ * engine's stream, or as one kernel that advances each system inside a
+ * thread-block cluster: where every system of the engine has 2 to 4 cells and
+ * at least 5 list sub-cells per side (N = 460 to 4050 at density 1.2 and the
+ * default skin), thermostat 0, 1 or 2 and no uniform shuffle (shuffle 2), and
+ * its cluster's shared memory holds the largest; acg_get_run_plan tells.
+ * Returns after queuing (acg_sync waits). */
 int acg_step(acg_engine *e, int nsteps);
 /* The same steps launched kernel by kernel without a CUDA graph (every
  * rebuild kernel is launched and skips the systems that need no rebuild). */
@@ -338,6 +341,15 @@ int acg_set_group_tpp(acg_engine *e, int gtpp);
  * the reference. */
 int acg_set_box_cells(acg_engine *e, int cells);
 int acg_get_box_cells(acg_engine *e, int *cells);
+
+/* How acg_step advances the engine: *cluster = blocks of the thread-block
+ * cluster that holds each system (0: the engine steps kernel by kernel),
+ * *threads = threads per block, *resident = 1 where a block keeps its
+ * particles' state in shared memory; calls of fewer than *min_steps steps go
+ * kernel by kernel all the same, and one launch takes at most *max_steps
+ * steps.  Results do not depend on any of it.  Any pointer may be NULL.  No
+ * counterpart in the reference. */
+int acg_get_run_plan(acg_engine *e, int *cluster, int *threads, int *resident, int *min_steps, int *max_steps);
 
 const char *acg_last_error(void);
 const char *acg_version(void);
