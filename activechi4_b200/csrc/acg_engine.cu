@@ -251,6 +251,7 @@ struct acg_engine {
   // steps kernel by kernel), state in shared memory, dynamic shared memory,
   // systems in launch order (device)
   int run_c = 0, run_resident = 0;
+  int run_min = 1;  // fewest steps of a call that runs this way
   size_t run_smem = 0;
   int *run_order = nullptr;
   int2 *d_tiles_b = nullptr;
@@ -394,6 +395,22 @@ void plan_run(acg_engine *e, size_t smem_limit) {
     if (least > smem_limit) continue;
     e->run_c = C;
     e->run_resident = resident;
+    // Short calls of many systems go kernel by kernel.  A cluster that rebuilds
+    // its lists takes several steps' time for it, and with a few dozen systems
+    // one or another does nearly every step: a call waits for it where longer
+    // calls average over them, while the kernels share its work among all SMs.
+    // Both paths give the same bits.  Measured, us a step in calls of 1, 2, 4 and
+    // 8 steps, in clusters / kernel by kernel, by the largest system's particles
+    // per block (FP32; FP64 crosses at the same places or before):
+    //   250 (N = 1000, 16 systems)   87 / 112
+    //   500 (N = 2000, 16 systems)  152 / 123,  96 / 111
+    //  1000 (N = 2000, 34 systems)  338 / 153, 194 / 142, 117 / 140
+    //  2000 (N = 4000, 34 systems)  486 / 192, 298 / 187, 185 / 185, 128 / 177
+    //  4000 (N = 4000, 75 systems)  902 / 293, 525 / 281, 335 / 277, 237 / 273
+    int n_max = 0;
+    for (const SysDesc &d : L.desc) n_max = std::max(n_max, d.n);
+    const int load = (n_max + C - 1) / C;
+    e->run_min = load <= 250 ? 1 : 1 + (load + 499) / 500 + (load > 500);
     e->run_smem = std::min(smem_limit, std::max(least, want));
     return;
   }
@@ -411,6 +428,9 @@ void run_config(const acg_engine *e, cudaLaunchConfig_t &cfg, cudaLaunchAttribut
   cfg.attrs = &at;
   cfg.numAttrs = 1;
 }
+
+// whether a call of nsteps steps runs inside clusters
+bool takes_run(const acg_engine *e, long long nsteps) { return e->run_c && nsteps >= e->run_min; }
 
 // nsteps steps of every system, one cluster each
 int launch_run(acg_engine *e, int nsteps) {
@@ -1696,10 +1716,11 @@ int acg_compute_forces(acg_engine *e) {
   return ACG_OK;
 }
 
-// nsteps steps in graph launches (no drift removal due inside them)
-int step_graphs(acg_engine *e, int nsteps) {
+// nsteps steps in graph launches, or inside clusters (`run`); no drift removal is
+// due inside them
+int step_graphs(acg_engine *e, int nsteps, bool run) {
   int rc;
-  if (e->run_c) {
+  if (run) {
     // launches of bounded length, so other engines' work gets the SMs between them
     for (int left = nsteps; left > 0; left -= std::min(left, RUN_STEPS)) {
       rc = launch_run(e, std::min(left, RUN_STEPS));
@@ -1755,7 +1776,7 @@ int acg_step(acg_engine *e, int nsteps) {
   int rc = prime(e);
   if (rc) return rc;
   for (const auto &pc : drift_pieces(e, e->hstep, e->hramp, nsteps)) {
-    rc = step_graphs(e, (int)pc.first);
+    rc = step_graphs(e, (int)pc.first, takes_run(e, nsteps));
     if (rc) return rc;
     if (pc.second) {
       rc = launch_drift(e);
@@ -1770,8 +1791,10 @@ int acg_prepare(acg_engine *e) {
   CK(cudaSetDevice(e->device));
   int rc = prime(e);
   if (rc) return rc;
-  if (e->no_while || e->run_c) return ACG_OK;
-  for (int k = 0; k < 3 && !e->no_while; k++)
+  // an engine that runs inside clusters takes the one-step graph for its short
+  // calls (up to 18 steps) alone
+  if (e->no_while || (e->run_c && e->run_min <= 1)) return ACG_OK;
+  for (int k = e->run_c ? 2 : 0; k < 3 && !e->no_while; k++)
     if (!e->wexec[k] &&
         build_while_graph(e, k < 2 ? GRAPH_STEPS : 1, e->counts + k, &e->wgraph[k], &e->wexec[k]) != ACG_OK)
       e->no_while = true;
@@ -1955,7 +1978,7 @@ int acg_get_run_plan(acg_engine *e, int *cluster, int *threads, int *resident, i
   if (cluster) *cluster = e->run_c;
   if (threads) *threads = run ? run_threads(e->lay.desc[0].precision, e->run_resident) : 0;
   if (resident) *resident = run && e->run_resident;
-  if (min_steps) *min_steps = run ? 1 : 0;
+  if (min_steps) *min_steps = run ? e->run_min : 0;
   if (max_steps) *max_steps = run ? RUN_STEPS : 0;
   return ACG_OK;
 }
@@ -2126,6 +2149,7 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
   CK(cudaSetDevice(e->device));
   int rc = prime(e);
   if (rc) return rc;
+  const bool run = takes_run(e, nsteps);
   // exactly nsteps steps: one graph of nsteps steps when that is short, else
   // graphs of GRAPH_STEPS steps and one of the remainder
   std::vector<int> plan;
@@ -2145,7 +2169,7 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
   for (const auto &reg : pieces)
     for (const auto &pc : reg) {
       const int K = (int)pc.first;
-      if (e->run_c || e->bench.count(K)) continue;
+      if (run || e->bench.count(K)) continue;
       cudaGraph_t g;
       cudaGraphExec_t x;
       rc = build_graph(e, K, &g, &x);
@@ -2174,7 +2198,7 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
     if (flush_bytes) CK(cudaMemsetAsync(e->flush, (int)(c & 0xff), flush_bytes, e->stream));
     CK(cudaEventRecord(ev[2 * c], e->stream));
     for (const auto &pc : pieces[c]) {
-      if (e->run_c) {
+      if (run) {
         rc = launch_run(e, (int)pc.first);
         if (rc) return rc;
         nrun++;
@@ -2201,7 +2225,7 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
   CK(cudaMemcpy(st1.data(), e->v.st, sizeof(SysState) * nsys, cudaMemcpyDeviceToHost));
   *ms = tot;
   if (!launches) return ACG_OK;
-  if (e->run_c) {  // whole runs in one launch, and the drift removals
+  if (run) {  // whole runs in one launch, and the drift removals
     *launches = nrun + 2 * ndrift;
     return ACG_OK;
   }
