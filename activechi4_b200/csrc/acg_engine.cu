@@ -35,7 +35,9 @@ int fail(int code, const std::string &msg) {
 
 constexpr double TAU_T = 0.20;  // MDcode/time_evolve.c:477
 constexpr int GRAPH_STEPS = 32;
-constexpr int RUN_STEPS = 2048;       // most steps of one k_run_box launch (tens of ms)
+constexpr int RUN_STEPS = 2048;       // most steps of one k_run_box launch
+constexpr double RUN_FULL_US = 12e3;  // about the longest one may take that occupies the whole chip
+constexpr int RUN_FULL_STEPS = 16;    // ... but no fewer steps than this
 constexpr int BENCH_MAX_GRAPH = 256;  // acg_bench_steps: one graph for up to this many steps
 
 struct Layout {
@@ -252,6 +254,7 @@ struct acg_engine {
   // systems in launch order (device)
   int run_c = 0, run_resident = 0;
   int run_min = 1;  // fewest steps of a call that runs this way
+  int run_max = RUN_STEPS;  // most steps of one launch
   size_t run_smem = 0;
   int *run_order = nullptr;
   int2 *d_tiles_b = nullptr;
@@ -373,7 +376,7 @@ bool run_eligible(const SysDesc &d) { return d.box && d.msub >= 5 && d.thermosta
 // as leave every system its own cluster on the chip at once (7 of 16 blocks,
 // 15 of 8, 33 of 4, 74 of 2 with one block per SM), then one block per system;
 // more where a system does not fit otherwise.
-void plan_run(acg_engine *e, size_t smem_limit) {
+void plan_run(acg_engine *e, size_t smem_limit, int nsm) {
   const Layout &L = e->lay;
   e->run_c = 0;
   for (int r = 0; r < L.nsys; r++)
@@ -395,6 +398,7 @@ void plan_run(acg_engine *e, size_t smem_limit) {
     if (least > smem_limit) continue;
     e->run_c = C;
     e->run_resident = resident;
+    e->run_smem = std::min(smem_limit, std::max(least, want));
     // Short calls of many systems go kernel by kernel.  A cluster that rebuilds
     // its lists takes several steps' time for it, and with a few dozen systems
     // one or another does nearly every step: a call waits for it where longer
@@ -411,7 +415,24 @@ void plan_run(acg_engine *e, size_t smem_limit) {
     for (const SysDesc &d : L.desc) n_max = std::max(n_max, d.n);
     const int load = (n_max + C - 1) / C;
     e->run_min = load <= 250 ? 1 : 1 + (load + 499) / 500 + (load > 500);
-    e->run_smem = std::min(smem_limit, std::max(least, want));
+    // Clusters that occupy (nearly) every SM keep all other work off the chip
+    // until systems finish, so their launches are cut to about RUN_FULL_US (a step
+    // is estimated as 8 us and 0.05 us, FP64 0.075, for each particle that a block
+    // steps in turn: within 15 % from N = 1000 on 16 blocks to 200 of 4000).
+    // Measured with a batch of 256 replicas (FP32, 500 to 4000 particles, 1024
+    // steps) and 32 steps of a run of N = 11154 on another stream beside it, ms for
+    // the batch and for the run, by the steps of a launch: 2048 256 and 215, 128 255
+    // and 26, 64 256 and 12, 32 261 and 11, 16 272 and 12, 8 276 and 11; kernel by
+    // kernel 419 and 5.  (Shorter launches wait for the slowest system's list
+    // rebuild more often.)  Where SMs are left over the run takes 3 ms whatever the
+    // launches' length: 75 systems of one block each, 7 of 16.
+    long long total = 0;
+    for (const SysDesc &d : L.desc) total += d.n;
+    const int blocks = L.nsys * C, waves = (blocks + nsm - 1) / nsm;
+    if (10 * blocks > 9 * nsm) {
+      const double us = 8.0 + (prec ? 0.05 : 0.075) * std::max((double)load, (double)waves * total / blocks);
+      e->run_max = std::max(RUN_FULL_STEPS, (int)std::min((double)RUN_STEPS, RUN_FULL_US / us));
+    }
     return;
   }
 }
@@ -1221,7 +1242,7 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
     return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)need) == cudaSuccess;
   };
   bool attr_ok = true;
-  plan_run(e, RUN_SMEM_MAX);
+  plan_run(e, RUN_SMEM_MAX, nsm);
   if (e->run_c) {
     std::vector<int> ord(nsys);
     for (int r = 0; r < nsys; r++) ord[r] = r;
@@ -1721,10 +1742,13 @@ int acg_compute_forces(acg_engine *e) {
 int step_graphs(acg_engine *e, int nsteps, bool run) {
   int rc;
   if (run) {
-    // launches of bounded length, so other engines' work gets the SMs between them
-    for (int left = nsteps; left > 0; left -= std::min(left, RUN_STEPS)) {
-      rc = launch_run(e, std::min(left, RUN_STEPS));
+    // launches of bounded and about equal length, so other engines' work gets the
+    // SMs between them
+    for (int left = nsteps, pieces = (nsteps + e->run_max - 1) / e->run_max; left > 0; pieces--) {
+      const int k = (left + pieces - 1) / pieces;
+      rc = launch_run(e, k);
       if (rc) return rc;
+      left -= k;
     }
     return ACG_OK;
   }
@@ -1979,7 +2003,7 @@ int acg_get_run_plan(acg_engine *e, int *cluster, int *threads, int *resident, i
   if (threads) *threads = run ? run_threads(e->lay.desc[0].precision, e->run_resident) : 0;
   if (resident) *resident = run && e->run_resident;
   if (min_steps) *min_steps = run ? e->run_min : 0;
-  if (max_steps) *max_steps = run ? RUN_STEPS : 0;
+  if (max_steps) *max_steps = run ? e->run_max : 0;
   return ACG_OK;
 }
 
