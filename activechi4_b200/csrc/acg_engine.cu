@@ -332,6 +332,9 @@ size_t shuffle_smem(const Layout &lay) {
 }
 size_t sort_sub_smem(int nmax, int m3max) { return (size_t)nmax * 2 * sizeof(uint16_t) + (2 * (size_t)m3max + 1) * sizeof(int); }
 
+using ListFn = void (*)(View);
+ListFn box_list_fn(const View &v) { return v.box_warp ? k_build_list_box<true> : k_build_list_box<false>; }
+
 ForceFn force_fn(int tpp, int prec) {
 #define F(T)                                                                     \
   case T:                                                                        \
@@ -575,9 +578,9 @@ void drop_graphs(acg_engine *e) {
 // memory) and can be updated in place instead of instantiated anew
 std::string graph_shape(const acg_engine *e, int K) {
   char b[160];
-  snprintf(b, sizeof(b), "K%d g%d x%d b%d l%d%d p%d t%d/%d/%d/%d i%d%d%d", K, e->ntiles_g > 0, e->ntiles_x > 0,
+  snprintf(b, sizeof(b), "K%d g%d x%d b%d l%d%d p%d t%d/%d/%d/%d i%d%d%d w%d", K, e->ntiles_g > 0, e->ntiles_x > 0,
            e->ntiles_b > 0, e->ntiles_l > 0, e->ntiles_lc > 0, e->lay.desc[0].precision, e->tpp, e->gtpp, e->btpp, e->block,
-           e->any_gauss, e->any_npt, e->any_brown);
+           e->any_gauss, e->any_npt, e->any_brown, e->v.box_warp);
   return b;
 }
 
@@ -639,7 +642,7 @@ int launch_rebuild(acg_engine *e) {
   // the list build reads the compacted rebuild list whenever it runs
   if (e->ntiles_x) k_rebuild_compact<<<1, BLOCK_COMPACT, 0, s>>>(v);
   if (e->ntiles_g) k_build_list_groups<<<e->ntiles_g, BLOCK_G, list_smem(v.gcap), s>>>(v);
-  if (e->ntiles_x) k_build_list_box<<<e->ntiles_x * LIST_SPLIT, BLOCK_X, box_list_smem(e->lay.box_cell_nmax), s>>>(v);
+  if (e->ntiles_x) box_list_fn(v)<<<e->ntiles_x * LIST_SPLIT, BLOCK_X, box_list_smem(e->lay.box_cell_nmax), s>>>(v);
   if (e->ntiles_lc) k_build_list_cells<<<e->ntiles_lc, BLOCK_LC, list_cells_smem(v.lccap), s>>>(v);
   if (e->ntiles_l) k_build_list<<<e->ntiles_l, BLOCK_L, 0, s>>>(v);
   CK(cudaGetLastError());
@@ -864,7 +867,7 @@ int add_steps(acg_engine *e, cudaGraph_t g, int K, cudaGraphNode_t *prev_io) {
                sort_sub_smem(e->lay.box_nmax, e->lay.box_m3max)},
               {(void *)k_rebuild_compact, e->ntiles_x ? 1 : 0, BLOCK_COMPACT, 0},
               {(void *)k_build_list_groups, e->ntiles_g, BLOCK_G, list_smem(v.gcap)},
-              {(void *)k_build_list_box, e->ntiles_x * LIST_SPLIT, BLOCK_X, box_list_smem(e->lay.box_cell_nmax)},
+              {(void *)box_list_fn(v), e->ntiles_x * LIST_SPLIT, BLOCK_X, box_list_smem(e->lay.box_cell_nmax)},
               {(void *)k_build_list_cells, e->ntiles_lc, BLOCK_LC, list_cells_smem(v.lccap)},
               {(void *)k_build_list, e->ntiles_l, BLOCK_L, 0}};
     int all = -1, sbytes = (int)shuffle_smem(e->lay);
@@ -1277,7 +1280,7 @@ int acg_create(const acg_params *params, int nsys, int device, acg_engine **out)
     }
     for (int gt : {1, 2, 4})
       for (int pr : {0, 1}) attr_ok = attr_ok && raise_smem((const void *)box_fn(gt, pr), box_smem(L.box_nmax, pr));
-    attr_ok = attr_ok && raise_smem((const void *)k_build_list_box, box_list_smem(L.box_cell_nmax));
+    attr_ok = attr_ok && raise_smem((const void *)box_list_fn(v), box_list_smem(L.box_cell_nmax));
     attr_ok = attr_ok && raise_smem((const void *)k_sort_sub, sort_sub_smem(L.box_nmax, L.box_m3max));
   }
   // threads per particle of the whole-box kernels: fixed (not derived from the
