@@ -453,8 +453,12 @@ void run_config(const acg_engine *e, cudaLaunchConfig_t &cfg, cudaLaunchAttribut
   cfg.numAttrs = 1;
 }
 
-// whether a call of nsteps steps runs inside clusters
-bool takes_run(const acg_engine *e, long long nsteps) { return e->run_c && nsteps >= e->run_min; }
+// whether a call of nsteps steps, in so many pieces (cut where drift removals are
+// due), runs inside clusters: the pieces are launches of their own, so it is their
+// mean length that has to reach run_min
+bool takes_run(const acg_engine *e, long long nsteps, size_t pieces) {
+  return e->run_c && nsteps >= e->run_min * (long long)pieces;
+}
 
 // nsteps steps of every system, one cluster each
 int launch_run(acg_engine *e, int nsteps) {
@@ -1802,8 +1806,10 @@ int acg_step(acg_engine *e, int nsteps) {
   CK(cudaSetDevice(e->device));
   int rc = prime(e);
   if (rc) return rc;
-  for (const auto &pc : drift_pieces(e, e->hstep, e->hramp, nsteps)) {
-    rc = step_graphs(e, (int)pc.first, takes_run(e, nsteps));
+  const auto pieces = drift_pieces(e, e->hstep, e->hramp, nsteps);
+  const bool run = takes_run(e, nsteps, pieces.size());
+  for (const auto &pc : pieces) {
+    rc = step_graphs(e, (int)pc.first, run);
     if (rc) return rc;
     if (pc.second) {
       rc = launch_drift(e);
@@ -2176,7 +2182,6 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
   CK(cudaSetDevice(e->device));
   int rc = prime(e);
   if (rc) return rc;
-  const bool run = takes_run(e, nsteps);
   // exactly nsteps steps: one graph of nsteps steps when that is short, else
   // graphs of GRAPH_STEPS steps and one of the remainder
   std::vector<int> plan;
@@ -2193,6 +2198,9 @@ int acg_bench_steps(acg_engine *e, int64_t nsteps, size_t flush_bytes, double *m
     std::vector<long long> hs = e->hstep, hr = e->hramp;
     for (int K : plan) pieces.push_back(drift_pieces(e, hs, hr, K));
   }
+  size_t npieces = 0;
+  for (const auto &reg : pieces) npieces += reg.size();
+  const bool run = takes_run(e, nsteps, npieces);
   for (const auto &reg : pieces)
     for (const auto &pc : reg) {
       const int K = (int)pc.first;
