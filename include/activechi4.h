@@ -242,8 +242,9 @@ int acg_compute_forces(acg_engine *e);
  * engine's stream, or as one kernel that advances each system inside a
  * thread-block cluster: where every system of the engine has 2 to 4 cells and
  * at least 5 list sub-cells per side (N = 460 to 4050 at density 1.2 and the
- * default skin), thermostat 0, 1 or 2 and no uniform shuffle (shuffle 2), and
- * its cluster's shared memory holds the largest; acg_get_run_plan tells.
+ * default skin), thermostat 0, 1 or 2 and no uniform shuffle (shuffle 2),
+ * nb_capacity is not below the mean neighbour count, and a cluster's shared
+ * memory holds the largest; acg_get_run_plan tells.
  * Returns after queuing (acg_sync waits). */
 int acg_step(acg_engine *e, int nsteps);
 /* The same steps launched kernel by kernel without a CUDA graph (every
