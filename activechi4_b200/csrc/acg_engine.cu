@@ -412,9 +412,10 @@ void plan_run(acg_engine *e, size_t smem_limit, int nsm) {
     // its lists takes several steps' time for it, and with a few dozen systems
     // one or another does nearly every step: a call waits for it where longer
     // calls average over them, while the kernels share its work among all SMs.
-    // Both paths give the same bits.  Measured, us a step in calls of 1, 2, 4 and
-    // 8 steps, in clusters / kernel by kernel, by the largest system's particles
-    // per block (FP32; FP64 crosses at the same places or before):
+    // Both paths give the same bits.  The line lies where the two meet, between
+    // these (us a step in calls of 1, 2, 4 and 8 steps, in clusters / kernel by
+    // kernel, by the largest system's particles per block; FP32, FP64 meets there
+    // or before):
     //   250 (N = 1000, 16 systems)   87 / 112
     //   500 (N = 2000, 16 systems)  152 / 123,  96 / 111
     //  1000 (N = 2000, 34 systems)  338 / 153, 194 / 142, 117 / 140
@@ -423,7 +424,7 @@ void plan_run(acg_engine *e, size_t smem_limit, int nsm) {
     int n_max = 0;
     for (const SysDesc &d : L.desc) n_max = std::max(n_max, d.n);
     const int load = (n_max + C - 1) / C;
-    e->run_min = load <= 250 ? 1 : 1 + (load + 499) / 500 + (load > 500);
+    e->run_min = load <= 250 ? 1 : 1 + (3 * load + 1999) / 2000;
     // Clusters that occupy (nearly) every SM keep all other work off the chip
     // until systems finish, so their launches are cut to about RUN_FULL_US (a step
     // is estimated as 8 us and 0.05 us, FP64 0.075, for each particle that a block
@@ -1831,7 +1832,7 @@ int acg_prepare(acg_engine *e) {
   int rc = prime(e);
   if (rc) return rc;
   // an engine that runs inside clusters takes the one-step graph for its short
-  // calls (up to 18 steps) alone
+  // calls (up to 13 steps) alone
   if (e->no_while || (e->run_c && e->run_min <= 1)) return ACG_OK;
   for (int k = e->run_c ? 2 : 0; k < 3 && !e->no_while; k++)
     if (!e->wexec[k] &&

@@ -12,7 +12,7 @@ pytestmark = pytest.mark.gpu
 
 @pytest.mark.parametrize("sizes,min_steps", [
     ([1000] * 7, 1), ([4000], 1), ([2000] * 8, 1), ([4000] * 8, 2), ([1000] * 33, 1), ([2000] * 16, 2), ([500] * 34, 1),
-    ([1000] * 34, 2), ([2000] * 34, 4), ([4000] * 34, 6), ([500] * 75, 2), ([1000] * 75, 4)])
+    ([1000] * 34, 2), ([2000] * 34, 3), ([4000] * 34, 4), ([500] * 75, 2), ([1000] * 75, 3), ([4000] * 75, 7)])
 @pytest.mark.parametrize("precision", [0, 1])
 def test_line(cuda_lib, sizes, min_steps, precision):
     from activechi4_b200 import Engine, default_params
