@@ -47,9 +47,9 @@ constexpr int LIST_SPLIT = 4;     // blocks sharing a whole-box tile in the list
 constexpr double BRICK2_MAX = ACG_BRICK2_MAX;
 // whole-box particles up to which the list kernel builds lists one warp per
 // particle (the few systems that rebuild in a step are done sooner; us a step of
-// the kernel-by-kernel path, FP32, per particle / by bricks: one of N = 1000 43 /
-// 44, of N = 4000 59 / 61, 16 of 1000 84 / 96, 8 of 2000 76 / 81, 4 of 4000 77 /
-// 80; 8 of 4000 98 / 98)
+// the kernel-by-kernel path, FP32, per particle / by bricks: one of N = 4000 56 /
+// 58, 16 of 1000 83 / 99, 8 of 2000 76 / 84, 4 of 4000 75 / 82; from 8 of 4000 on
+// they meet)
 constexpr int BOX_WARP_MAX = 16384;
 constexpr int GSPLIT_MAX = 8;     // most force blocks per cell group (small boxes)
 // measured on B200 (FP32, T = 0.45, step latency of one system alone):

@@ -1079,8 +1079,9 @@ __device__ __forceinline__ double4 total_of_segments(const double4 *seg, int nse
 // thermostat chain (runs in a single block).  The system's state and
 // descriptor are copied to shared memory beside the partial sums (one round
 // trip to L2) and the state is written back whole, so the one thread that
-// runs the chain waits for no memory.  seg: shared memory for a whole-box
-// system's segment sums (32 bytes per 32 slots).
+// runs the chain waits for no memory.  BOX: a whole-box system; seg: shared memory
+// for its segment sums (32 bytes per 32 slots).
+template <bool BOX>
 __device__ void finalize_system(const View &v, int r, int mode, double4 *seg) {
   __shared__ double sh[4][32];
   __shared__ SysState ss;
@@ -1090,7 +1091,7 @@ __device__ void finalize_system(const View &v, int r, int mode, double4 *seg) {
   copy_struct(&sd, &v.desc[r]);
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = blockDim.x >> 5;
   double4 t = make_double4(0.0, 0.0, 0.0, 0.0);
-  if (dg.box) {
+  if (BOX) {
     const int n = dg.n, nseg = (n + 31) >> 5;
     constexpr int F = 4;  // segments in flight a warp (one at a time the FP32 force kernel of N = 4000 took 24.6 us, so 22.6)
     for (int g0 = w; g0 < nseg; g0 += F * nw) {
@@ -1963,7 +1964,7 @@ __global__ void __launch_bounds__(512) k_force_kick(View v, int mode, int tile_b
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  finalize_system(v, r, mode, nullptr);
+  finalize_system<false>(v, r, mode, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -2462,13 +2463,14 @@ __device__ __forceinline__ void particle_epilogue(const V &v, const SysDesc &d, 
 
 // block sums stored at the block's partial slot of the system; the last block
 // of the system to finish (a counter, no waiting) finalises it
+template <bool BOX>
 __device__ __forceinline__ void end_force_block(const View &v, int r, int slot, int mode, double pe, double vir,
                                                 double ke, double va, double4 *seg) {
   __shared__ double sh[32];
   __shared__ int s_last;
   const SysDesc &d = v.desc[r];
   SysState &st = v.st[r];
-  if (!d.box) {
+  if (!BOX) {
     pe = block_sum_dyn(pe, sh);
     vir = block_sum_dyn(vir, sh);
     ke = block_sum_dyn(ke, sh);
@@ -2478,14 +2480,14 @@ __device__ __forceinline__ void end_force_block(const View &v, int r, int slot, 
     __syncthreads();
   }
   if (threadIdx.x == 0) {
-    if (!d.box) v.part_b[d.tile0_b + slot] = make_double4(pe, vir, ke, va);
+    if (!BOX) v.part_b[d.tile0_b + slot] = make_double4(pe, vir, ke, va);
     __threadfence();
     s_last = atomicAdd(&st.counter_b, 1u) == (unsigned)(d.ntile_b - 1);
   }
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  finalize_system(v, r, mode, seg);
+  finalize_system<BOX>(v, r, mode, seg);
 }
 
 template <int TPP, int PREC>
@@ -2676,7 +2678,7 @@ __global__ void __launch_bounds__(BLOCK_G, PREC ? ACG_FORCE_MINB32 : ACG_FORCE_M
     if (!valid || lane != 0) continue;
     particle_epilogue(v, d, st, i, mode, a, pe, vir, ke, va);
   }
-  end_force_block(v, r, tile.y, mode, pe, vir, ke, va, nullptr);
+  end_force_block<false>(v, r, tile.y, mode, pe, vir, ke, va, nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -3257,7 +3259,7 @@ __global__ void __launch_bounds__(BLOCK_COMPACT) k_rebuild_compact(View v) {
 // warps, each block staging the system once.
 // WARP: v.box_warp as a constant (the bricks' buffers in shared memory leave the
 // lists of one particle a warp, which read the sorted system through L1, next to
-// no L1: 16 systems of N = 1000 rebuilt in 236 us against 154 without them)
+// no L1: 16 systems of N = 1000 rebuilt in 187 us with them, 167 without)
 template <bool WARP>
 __global__ void __launch_bounds__(BLOCK_X) k_build_list_box(View v) {
   extern __shared__ float4 xstg[];
@@ -3452,7 +3454,7 @@ __global__ void __launch_bounds__(BLOCK_X, 4) k_force_box(View v, int mode) {
     particle_epilogue(v, d, st, i, mode, a, pei, viri, kei, vai);
     v.pacc[i] = make_double4(pei, viri, kei, vai);
   }
-  end_force_block(v, r, b, mode, 0.0, 0.0, 0.0, 0.0, reinterpret_cast<double4 *>(xsm));
+  end_force_block<true>(v, r, b, mode, 0.0, 0.0, 0.0, 0.0, reinterpret_cast<double4 *>(xsm));
 }
 
 // ---------------------------------------------------------------------------
