@@ -142,16 +142,14 @@ class Server:
         if self.priority == "size":
             return int(np.clip(2.0 * (math.log10(req.n) - 3.0), 0, 4))
         if self.priority == "time":
-            # expected device time alone: a step costs at least ~45 us (kernel
-            # latency) and about 1 ns per particle beyond that
-            est = req.steps * max(45e-6, 1.0e-9 * req.n)
+            est = req.steps * step_seconds(req.n)
             return int(np.clip(np.floor(np.log2(max(est, 1.0))), 0, 4))
         return 0
 
     def _chunk(self, n, left):
-        # about chunk_work particle-steps, and no more than ~20 ms of device
-        # time for small systems, whose steps cost ~50 us whatever their size
-        k = min(self.chunk_work / max(n, 1), 0.02 / 5e-5)
+        # about chunk_work particle-steps, and no more than 400 steps of small
+        # systems (5 to 20 ms of device time)
+        k = min(self.chunk_work / max(n, 1), 400)
         k = int(max(32, min(8192, round(k / 32) * 32)))
         return min(k, left)
 
@@ -263,6 +261,16 @@ def poisson_requests(count, rate=20.0, n_range=(1000, 256000), step_range=(10000
         reqs.append(RunRequest(i, n, max(64, steps), float(rng.choice(T_SET)), float(rng.choice(F0_SET)),
                                int(rng.choice(TAU_SET)), seed=10000 * seed + i, arrival=t, precision=precision))
     return reqs
+
+
+def step_seconds(n: int) -> float:
+    """Expected device time of one FP32 step of a run alone on the GPU: inside a
+    cluster up to about 4050 particles (11.5 us at N = 1000, 20 at 4000), bound by
+    kernel latency up to 20000 (29 us at 4100, 36 at 16000), about 1 ns a particle
+    in large systems (74 us at 50000, 98 at 100000, 240 at 256000)."""
+    if n < 4050:
+        return 8.7e-6 + 2.8e-9 * n
+    return max(26e-6 + 0.75e-9 * n, 0.93e-9 * n)
 
 
 def next_admissible(queue, active_n, max_big=None, big_n=20000) -> int:
