@@ -6,10 +6,13 @@ Used as the command under Nsight Compute; prints nothing but a summary line.
   python -m activechi4_b200.profile_case --stage step --n 100000 --reps 64
 
   python -m activechi4_b200.profile_case --stage step --replicas 256 --reps 64
+  python -m activechi4_b200.profile_case --stage run --n 1000 --reps 64
 
 Stages: force (pair forces only, the force kernel's work), rebuild (cell
 build + neighbour lists at the current positions), step (whole timesteps,
-launched kernel by kernel so each launch is listed separately), latency (no
+launched kernel by kernel so each launch is listed separately), run (one acg_step
+call: the cluster kernel where the engine takes it), noalloc (the allocation-free
+forces of one system off the lattice), latency (no
 profiler: one system at T = 0.45 from a lattice, NHC, 200 steps, then the
 step time of the production graphs over 640 steps and the kick/drift, force
 and rebuild stages alone, CUDA events; prints one JSON line).  The state is
@@ -30,7 +33,7 @@ from activechi4_b200.init import lattice_state
 
 def main():
     ap = argparse.ArgumentParser()
-    ap.add_argument("--stage", default="force", choices=["force", "rebuild", "step", "latency"])
+    ap.add_argument("--stage", default="force", choices=["force", "rebuild", "step", "run", "noalloc", "latency"])
     ap.add_argument("--n", type=int, default=100000)
     ap.add_argument("--reps", type=int, default=3)
     ap.add_argument("--melt", type=int, default=256)
@@ -44,6 +47,9 @@ def main():
     a = ap.parse_args()
     if a.stage == "latency":
         latency(a)
+        return
+    if a.stage == "noalloc":
+        noalloc(a)
         return
     if a.replicas:
         from activechi4_b200.batch import make_engine, replica_set
@@ -77,7 +83,7 @@ def main():
     elif a.stage == "rebuild":
         ms = e.time_stage(2, a.reps)
     else:
-        e.step_eager(a.reps)
+        (e.step if a.stage == "run" else e.step_eager)(a.reps)
         e.sync()
         ms = float("nan")
     cu.cuProfilerStop()
@@ -86,6 +92,32 @@ def main():
         th["rebuilds"] = sum(e.thermo(r)["rebuilds"] for r in range(e.nsys))
     print(f"stage={a.stage} n={a.n} replicas={a.replicas} reps={a.reps} ms/launch={ms:.4f} rebuilds={th['rebuilds']} "
           f"overflow={th['overflow']} launch={e.get_launch()}")
+
+
+def noalloc(a):
+    """`reps` calls of the allocation-free forces of one system off the lattice."""
+    import torch
+
+    from activechi4_b200 import _abi
+    st = lattice_state(a.n, 0.45, seed=3)
+    x = st.x + np.random.default_rng(3).uniform(-0.05, 0.05, st.x.shape) / st.L
+    x -= np.floor(x)
+    x[x >= 1.0] = 0.0
+    dev = torch.device("cuda")
+    arr = [torch.tensor(np.ascontiguousarray(v), device=dev) for v in (x, st.type, st.act_tag, st.k.reshape(-1))]
+    F, out = (torch.empty(s, dtype=torch.float64, device=dev) for s in ((a.n, 3), (3,)))
+    p = [ctypes.c_void_p(t.data_ptr()) for t in (*arr, F, out)]
+    cu = ctypes.CDLL("libcuda.so.1")
+    stream = ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    for k in range(3 + a.reps):
+        if k == 3:
+            torch.cuda.synchronize()
+            cu.cuProfilerStart()
+        _abi.check(_abi.lib().acg_forces_noalloc(p[0], None, p[1], p[2], p[3], a.n, st.nact, st.L, 1.0, p[4], p[5],
+                                                 stream))
+    torch.cuda.synchronize()
+    cu.cuProfilerStop()
+    print(f"stage=noalloc n={a.n} reps={a.reps} pe/n={float(out[0]) / a.n:.6f}")
 
 
 def latency(a):
