@@ -1,5 +1,5 @@
-"""Many independent replicas in one engine (small systems: one
-thread-block cluster each for a whole call; else one launch per kernel per step).
+"""Many independent replicas in one engine (where all are small: one thread-block
+cluster each for a whole call; else one launch per kernel per step).
 
 `replica_set` draws the replica parameters of the batched workload: N uniform
 in [n_min, n_max] with an 80:20 composition at density 1.2, T from

@@ -416,11 +416,11 @@ void plan_run(acg_engine *e, size_t smem_limit, int nsm) {
     // these (us a step in calls of 1, 2, 4 and 8 steps, in clusters / kernel by
     // kernel, by the largest system's particles per block; FP32, FP64 meets there
     // or before):
-    //   250 (N = 1000, 16 systems)   87 / 112
-    //   500 (N = 2000, 16 systems)  152 / 123,  96 / 111
-    //  1000 (N = 2000, 34 systems)  338 / 153, 194 / 142, 117 / 140
-    //  2000 (N = 4000, 34 systems)  486 / 192, 298 / 187, 185 / 185, 128 / 177
-    //  4000 (N = 4000, 75 systems)  902 / 293, 525 / 281, 335 / 277, 237 / 273
+    //   250 (N = 1000, 16 systems)   83 / 89
+    //   500 (N = 2000, 16 systems)  138 / 117,  89 / 106
+    //  1000 (N = 2000, 34 systems)  299 / 146, 176 / 139, 106 / 133
+    //  2000 (N = 4000, 34 systems)  490 / 189, 296 / 182, 184 / 175, 128 / 176
+    //  4000 (N = 4000, 75 systems)  894 / 292, 521 / 284, 333 / 278, 238 / 276
     int n_max = 0;
     for (const SysDesc &d : L.desc) n_max = std::max(n_max, d.n);
     const int load = (n_max + C - 1) / C;
@@ -431,9 +431,9 @@ void plan_run(acg_engine *e, size_t smem_limit, int nsm) {
     // steps in turn: within 15 % from N = 1000 on 16 blocks to 200 of 4000).
     // Measured with a batch of 256 replicas (FP32, 500 to 4000 particles, 1024
     // steps) and 32 steps of a run of N = 11154 on another stream beside it, ms for
-    // the batch and for the run, by the steps of a launch: 2048 256 and 215, 128 255
-    // and 26, 64 256 and 12, 32 261 and 11, 16 272 and 12, 8 276 and 11; kernel by
-    // kernel 419 and 5.  (Shorter launches wait for the slowest system's list
+    // the batch and for the run, by the steps of a launch: 2048 239 and 202, 128 238
+    // and 24, 64 238 and 11, 32 240 and 10, 16 256 and 8; kernel by kernel, before
+    // the cluster runs, 419 and 5.  (Shorter launches wait for the slowest system's list
     // rebuild more often.)  Where SMs are left over the run takes 3 ms whatever the
     // launches' length: 75 systems of one block each, 7 of 16.
     long long total = 0;

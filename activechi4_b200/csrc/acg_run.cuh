@@ -12,9 +12,9 @@
 //   * kick/drift: each block moves its slots, writes the new positions as staged
 //     to memory and its largest displacement into every block (distributed
 //     shared memory); cluster barrier; every block takes the same rebuild
-//     decision and reads all positions (storing them into the other 15 blocks
-//     took 6400 cycles at N = 4000 FP64, this 2000: one read is wide and
-//     coalesced, the remote stores are neither);
+//     decision and reads all positions (1400 cycles at N = 1000 and 3000 at N =
+//     4000, FP64, where storing them into the other 15 blocks took 2000 and 6400:
+//     one read is wide and coalesced, the remote stores are neither);
 //   * forces from the lists (kept in shared memory where they fit), second half
 //     kick, sums per 32 slots stored into every block; cluster barrier; every
 //     block adds them up in the same order and runs the thermostat chain.
@@ -25,13 +25,17 @@
 // per system, largest first, and no system waits for another's rebuild.  A list
 // rebuild happens inside the cluster: every block sorts the system by cell (a
 // stable counting sort over original indices, which gives the reference's
-// InCell order) and by list sub-cell in its shared memory, so only two cluster
-// barriers separate its phases.
+// InCell order) and by list sub-cell in its shared memory, so it takes two more
+// cluster barriers (a third where a list overflows).
 //
 // What bounds it: the latency of a step's dependent phases for a lone system
 // (16 of 148 SMs busy), the issue rate of the pair terms for a batch.  Measured
-// on B200 against the kernel-by-kernel graphs: N = 1000 FP64 39.0 -> 14.3 us a
-// step, N = 4000 FP64 60 -> 36, 256 FP32 replicas 400 -> 245.
+// on B200 against the kernel-by-kernel graphs it replaced, in calls of 64 steps of
+// a system just off the lattice: N = 1000 FP64 39.0 -> 14.3 us a step, N = 4000
+// FP64 60 -> 36, 256 FP32 replicas 400 -> 245; of settled systems N = 1000 13.5 us
+// (FP32 11.5), N = 4000 25.7 (20.0).  What it does worse than the kernels: a call
+// of a few steps of many systems, whose length is that of the slowest list rebuild
+// (such calls take the kernels).
 //
 // Sums, lists and particle order are those of the kernel-by-kernel step, so a
 // system's results are the same bits whichever path, cluster size or residency

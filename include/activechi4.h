@@ -227,12 +227,13 @@ int acg_set_barostat(acg_engine *e, int sys, const double *eta_baro3, const doub
 /* Change a system's thermostat temperature (and with it q). */
 int acg_set_temperature(acg_engine *e, int sys, double T);
 
-/* update_cell_list (MDcode/cell_list+forces.c:58-148) for every system:
+/* update_cell_list (MDcode/cell_list+forces.c:58-148) for every system that
+ * holds a state:
  * counting-sort cell build + neighbour lists. */
 int acg_rebuild(acg_engine *e);
 
-/* calculate_forces (MDcode/cell_list+forces.c:153-227) for every system at
- * the current positions (rebuilding cells/lists first when needed). */
+/* calculate_forces (MDcode/cell_list+forces.c:153-227) for every system that
+ * holds a state, at the current positions (rebuilding cells/lists first when needed). */
 int acg_compute_forces(acg_engine *e);
 
 /* Advance every system nsteps steps: for each step the direction shuffle
@@ -245,7 +246,8 @@ int acg_compute_forces(acg_engine *e);
  * default skin), thermostat 0, 1 or 2 and no uniform shuffle (shuffle 2),
  * nb_capacity is not below the mean neighbour count, and a cluster's shared
  * memory holds the largest; acg_get_run_plan tells.
- * Returns after queuing (acg_sync waits). */
+ * Returns after queuing (acg_sync waits).  A system that holds no state yet
+ * counts its steps and renews its directions, and nothing more. */
 int acg_step(acg_engine *e, int nsteps);
 /* The same steps launched kernel by kernel without a CUDA graph (every
  * rebuild kernel is launched and skips the systems that need no rebuild). */
