@@ -36,8 +36,8 @@ int fail(int code, const std::string &msg) {
 constexpr double TAU_T = 0.20;  // MDcode/time_evolve.c:477
 constexpr int GRAPH_STEPS = 32;
 constexpr int RUN_STEPS = 2048;       // most steps of one k_run_box launch
-constexpr double RUN_FULL_US = 12e3;  // about the longest one may take that occupies the whole chip
-constexpr int RUN_FULL_STEPS = 16;    // ... but no fewer steps than this
+constexpr double RUN_FULL_US = 20e3;  // about the longest one may take that occupies the whole chip
+constexpr int RUN_FULL_STEPS = 40;    // ... but no fewer steps than this
 constexpr int BENCH_MAX_GRAPH = 256;  // acg_bench_steps: one graph for up to this many steps
 
 struct Layout {
@@ -432,7 +432,7 @@ void plan_run(acg_engine *e, size_t smem_limit, int nsm) {
     // Measured with a batch of 256 replicas (FP32, 500 to 4000 particles, 1024
     // steps) and 32 steps of a run of N = 11154 on another stream beside it, ms for
     // the batch and for the run, by the steps of a launch: 2048 239 and 202, 128 238
-    // and 24, 64 238 and 11, 32 240 and 10, 16 256 and 8; kernel by kernel, before
+    // and 24, 85 (the bound) 237 and 14, 64 238 and 11, 32 240 and 10, 16 256 and 8; kernel by kernel, before
     // the cluster runs, 419 and 5.  (Shorter launches wait for the slowest system's list
     // rebuild more often.)  Where SMs are left over the run takes 3 ms whatever the
     // launches' length: 75 systems of one block each, 7 of 16.

@@ -22,7 +22,7 @@ def test_bound(cuda_lib, sizes, precision, full):
     k = min(k, 256)  # (acg_bench_steps times up to 256 steps in one launch)
     ms = min(e.bench_steps(k, 0)[0] for _ in range(3))
     # a launch of k steps (cut where a drift removal is due); the bound is an estimate: within a factor of two
-    assert k >= 16 and (ms < 24.0 or k == 16)
+    assert k >= 40 and (ms < 40.0 or k == 40)
 
 
 @pytest.mark.parametrize("precision", [0, 1])
@@ -30,7 +30,7 @@ def test_cut_calls(cuda_lib, precision):
     sizes = [460 + (37 * r) % 900 for r in range(150)]
     a, b = (_engine(sizes, precision) for _ in range(2))
     k = a.run_plan()["max_steps"]
-    assert 16 <= k < 400
+    assert 40 <= k < 700
     a.step(2 * k + 1)  # three launches
     b.step(k + 1)
     b.step(k)
