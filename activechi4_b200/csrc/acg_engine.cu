@@ -1758,9 +1758,10 @@ int step_graphs(acg_engine *e, int nsteps, bool run) {
   if (run) {
     // launches of bounded and about equal length, so other engines' work gets the
     // SMs between them
-    for (int left = nsteps, pieces = (nsteps + e->run_max - 1) / e->run_max; left > 0; pieces--) {
-      const int k = (left + pieces - 1) / pieces;
-      rc = launch_run(e, k);
+    long long left = nsteps;
+    for (long long pieces = (left + e->run_max - 1) / e->run_max; left > 0; pieces--) {
+      const long long k = (left + pieces - 1) / pieces;
+      rc = launch_run(e, (int)k);
       if (rc) return rc;
       left -= k;
     }
